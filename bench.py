@@ -364,11 +364,7 @@ def main():
     torch.cuda.synchronize()
     st_ms = {s: sum(a.elapsed_time(b) for a, b in st[s]) / K2 for s in st}
     dom = max((1, 2), key=lambda s: st_ms[s])
-    # FP64 sweep 1 runs the streaming kernel unless AINV_STREAM=0 forces the
-    # register family (AINV_STREAM=1 streams sweep 2 as well)
-    forced = os.environ.get("AINV_STREAM")
-    names = {1: "k_sweep_dscale" if forced == "0" else "k_stream_dscale",
-             2: "k_stream_axpby" if forced == "1" else "k_sweep_axpby"}
+    names = {1: "k_sweep_dscale", 2: "k_sweep_axpby"}
     dom_name = names[dom]
     peak, peak_kind = measured_peaks()
     PEAK[:] = [peak, peak_kind]

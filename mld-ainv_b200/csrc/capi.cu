@@ -333,9 +333,8 @@ int ainv_gpu_apply_stage(ainv_handle *h, char trans, int stage, double alpha,
   }
   cudaStream_t s = (cudaStream_t)stream;
   if (stage == 1)
-    return ainv::launch_sweep_dscale(tr ? h->zt : h->wt, h->d, x_dev, h->t, s, nullptr, h->status);
-  return ainv::launch_sweep_axpby(tr ? h->w : h->z, h->t, alpha, beta, y_dev, s, nullptr,
-                                  h->status);
+    return ainv::launch_sweep_dscale(tr ? h->zt : h->wt, h->d, x_dev, h->t, s);
+  return ainv::launch_sweep_axpby(tr ? h->w : h->z, h->t, alpha, beta, y_dev, s);
 }
 
 int ainv_gpu_apply_host(ainv_handle *h, char trans, double alpha, const double *x,
@@ -466,7 +465,7 @@ int ainv_csr_spmv(const ainv_csr *a, double alpha, const double *x_dev, double b
     ainv::set_error("ainv_csr_spmv: null argument");
     return AINV_ERR_ARG;
   }
-  return ainv::launch_spmv(a->a, alpha, x_dev, beta, y_dev, (cudaStream_t)stream, a->status);
+  return ainv::launch_spmv(a->a, alpha, x_dev, beta, y_dev, (cudaStream_t)stream);
 }
 
 int ainv_csr_destroy(ainv_csr *a) {

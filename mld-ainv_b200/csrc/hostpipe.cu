@@ -193,7 +193,7 @@ struct PipeLaunch {
   PipeArgs<V, T> a;
   int grid;
   cudaStream_t s;
-  template <int S, int P>
+  template <int P>
   void run() const {
     k_host_pipe<V, T, P><<<grid, kBlock, 0, s>>>(a);
   }
@@ -202,7 +202,7 @@ struct PipeLaunch {
 template <class V, class T>
 void launch_pipe(const DevSell &m1, const DevSell &m2, const PipeArgs<V, T> &a, int grid,
                  cudaStream_t s) {
-  with_pack<V, 1>(m1.pack, PipeLaunch<V, T>{a, grid, s});
+  with_pack<V>(m1.pack, PipeLaunch<V, T>{a, grid, s});
 }
 
 template <class V_, class T_>

@@ -106,6 +106,14 @@ struct DevSell {
   int *iptr = nullptr;  // nslices+1 index offsets (+16 bytes of tail padding)
   int *idx = nullptr;   // nidx offsets / columns (+16 bytes of tail padding)
   void *val = nullptr;  // slots, element type from prec
+  // One word group per slice, {sptr[s], start of its offsets in pidx (offset
+  // mode) or of its columns in idx, w, 1 in offset mode else 0}, and the
+  // distinct offset lists (a list that several slices share is stored once,
+  // so it stays in L1): a kernel that reads a slice through them has every
+  // value and gathered element of the slice one load away from its word group.
+  int4 *info = nullptr;  // nslices
+  int *pidx = nullptr;   // offset lists, each padded to a multiple of P
+  int wmax = 0;          // widest slice
   // streaming stages (see StageDesc); nstages = 0 when not streamable
   int nstages = 0;
   int stage_slices = 0;
@@ -196,22 +204,19 @@ namespace ainv {
 // t = d .* (M x) with M, d in prec; t is double (FP64) or float (mixed).
 // stop: optional device flag; when nonzero the kernel returns at once.
 int launch_sweep_dscale(const DevSell &m, const void *d, const double *x, void *t,
-                        cudaStream_t s, const int *stop = nullptr, int *status = nullptr);
+                        cudaStream_t s, const int *stop = nullptr);
 // y = alpha * M t + beta * y; t as produced by launch_sweep_dscale.
 int launch_sweep_axpby(const DevSell &m, const void *t, double alpha, double beta,
-                       double *y, cudaStream_t s, const int *stop = nullptr,
-                       int *status = nullptr);
-// The same two sweeps over the rows of slices [s0, s1) only (register path;
-// s0 a multiple of 4).  Rows outside the range are neither read nor written.
+                       double *y, cudaStream_t s, const int *stop = nullptr);
+// The same two sweeps over the rows of slices [s0, s1) only.  Rows outside
+// the range are neither read nor written.
 int launch_sweep_dscale_slices(const DevSell &m, const void *d, const double *x, void *t,
                                int s0, int s1, cudaStream_t s);
 int launch_sweep_axpby_slices(const DevSell &m, const void *t, double alpha, double beta,
                               double *y, int s0, int s1, cudaStream_t s);
 // y = alpha * A x + beta * y with an FP64 operator.
 int launch_spmv(const DevSell &a, double alpha, const double *x, double beta,
-                double *y, cudaStream_t s, int *status = nullptr);
-// Both sweeps of the apply for trans 'N' or 'T'/'C'.
-// status: device word for wait timeouts (the handle's own when null).
+                double *y, cudaStream_t s);
 // update_a (src/impl/mld_d_base_ainv_update_a.f90:53-79) on stream s:
 // d <- 1/(1/d_old + diag(W^T diag(x) Z)), d_old read from d64_in when given
 // (FP64) else from the handle's device d; the new d is stored in the
@@ -219,7 +224,7 @@ int launch_spmv(const DevSell &a, double alpha, const double *x, double beta,
 // d64_in.
 int update_a_async(ainv_handle *h, const double *x, const double *d64_in, double *d64,
                    cudaStream_t s);
+// Both sweeps of the apply for trans 'N' or 'T'/'C'.
 int ainv_apply_async(const ainv_handle *h, char trans, double alpha, const double *x,
-                     double beta, double *y, cudaStream_t s, const int *stop = nullptr,
-                     int *status = nullptr);
+                     double beta, double *y, cudaStream_t s, const int *stop = nullptr);
 }  // namespace ainv

@@ -20,7 +20,6 @@
 #include <cstdlib>
 #include <mutex>
 #include <map>
-#include <tuple>
 #include <utility>
 
 #include "stream.cuh"
@@ -30,55 +29,30 @@ namespace {
 
 using namespace dev;
 
-template <class V, class T, int S, int P>
-__global__ void __launch_bounds__(kBlock)
-    k_sweep_dscale(SellView<V> m, const double *__restrict__ x, const V *__restrict__ d,
-                   T *__restrict__ t, const int *__restrict__ stop) {
+// Slices [s0, s1) of a sweep (all of them, or a range of the host-array
+// pipeline).  HBM-bound: at 200^3 in FP64 sweep 1 moves 453 MB in 70.4 us and
+// sweep 2 389 MB in 60.7 us, 6.4 TB/s each.
+template <class V, class T, int P, int K>
+__global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
+    k_sweep_dscale(InfoView<V> m, const double *__restrict__ x, const V *__restrict__ d,
+                   T *__restrict__ t, int s0, int s1, const int *__restrict__ stop) {
   if (stop && *stop) return;
-  for_each_row<S, P>(m, x, [&](int row, auto acc) { t[row] = (T)(ldd(d + row) * acc); });
+  for_each_info<P, K>(
+      m, x, s0, s1, [&](int row) { return ldd(d + row); },
+      [&](int row, auto acc, auto dr) { t[row] = (T)(dr * acc); }, [](int) {});
 }
 
-// Every sweep-2 epilogue (register, slice-range, streaming and the host-array
-// pipeline kernels) uses axpby_row, so all forms give the same bits.
-template <class V, class T, int S, int P>
-__global__ void __launch_bounds__(kBlock)
-    k_sweep_axpby(SellView<V> m, const T *__restrict__ t, double alpha, double beta,
-                  double *__restrict__ y, const int *__restrict__ stop) {
+// Every sweep-2 epilogue (here and in the host-array pipeline kernel) uses
+// axpby_row, so all forms give the same bits.
+template <class V, class T, int P, int K>
+__global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
+    k_sweep_axpby(InfoView<V> m, const T *__restrict__ t, double alpha, double beta,
+                  double *__restrict__ y, int s0, int s1, const int *__restrict__ stop) {
   if (stop && *stop) return;
-  for_each_row<S, P>(m, t, [&](int row, auto acc) {
-    y[row] = axpby_row(alpha, (double)acc, beta, beta == 0.0 ? 0.0 : y[row]);
-  });
-}
-
-// Slice-range forms: groups [g0, g1) of S slices (the host-array pipeline).
-template <class V, class T, int S, int P>
-__global__ void __launch_bounds__(kBlock)
-    k_sweep_dscale_range(SellView<V> m, const double *__restrict__ x, const V *__restrict__ d,
-                         T *__restrict__ t, int g0, int g1) {
-  for_each_row<S, P>(
-      m, x, [&](int row, auto acc) { t[row] = (T)(ldd(d + row) * acc); }, g0, g1);
-}
-
-template <class V, class T, int S, int P>
-__global__ void __launch_bounds__(kBlock)
-    k_sweep_axpby_range(SellView<V> m, const T *__restrict__ t, double alpha, double beta,
-                        double *__restrict__ y, int g0, int g1) {
-  for_each_row<S, P>(
-      m, t,
-      [&](int row, auto acc) {
-        y[row] = axpby_row(alpha, (double)acc, beta, beta == 0.0 ? 0.0 : y[row]);
-      },
-      g0, g1);
-}
-
-// ---- streaming variants (stream.cuh) ----------------------------------------
-template <class V, class X, int P, class Epi>
-__global__ void __launch_bounds__(kStreamThreads, kStreamMinBlocks)
-    k_stream(SellView<V> m, const StageDesc *__restrict__ stages, int nstages,
-             const X *__restrict__ x, StreamLayout L, Epi epi, int *status,
-             const int *__restrict__ stop) {
-  if (stop && *stop) return;
-  stream_rows<P, stream_rmax<V>()>(m, stages, nstages, x, L, epi, status);
+  for_each_info<P, K>(
+      m, t, s0, s1, [&](int row) { return beta == 0.0 ? 0.0 : y[row]; },
+      [&](int row, auto acc, double yr) { y[row] = axpby_row(alpha, (double)acc, beta, yr); },
+      [](int) {});
 }
 
 inline int check_launch(const char *what) {
@@ -93,41 +67,6 @@ inline int check_launch(const char *what) {
 }  // namespace
 
 namespace dev {
-int group_size(int prec) {
-  static const int forced = [] {
-    const char *e = std::getenv("AINV_SLICES_PER_WARP");
-    const int v = e ? std::atoi(e) : 0;
-    return (v == 1 || v == 2 || v == 4) ? v : 0;
-  }();
-  if (forced) return forced;
-  return 2;
-}
-
-// Streaming (stream.cuh) is the default where it measured faster on B200 --
-// FP32 and BF16 factors, and sweep 1 (the D^-1 epilogue) of FP64 factors
-// (0.095 vs 0.102 ms at 200^3); FP64 sweep 2 (0.102 vs 0.086 ms) and the FP64
-// operator A use the register kernels.  Both families sum the same products
-// in the same slot order.  AINV_STREAM=0 / 1 forces one choice for every
-// matrix.
-namespace {
-int stream_forced() {
-  static const int forced = [] {
-    const char *e = std::getenv("AINV_STREAM");
-    return e ? (std::atoi(e) != 0 ? 1 : 0) : -1;
-  }();
-  return forced;
-}
-}  // namespace
-bool stream_enabled(int prec) {
-  if (stream_forced() >= 0) return stream_forced() == 1;
-  return prec != AINV_PREC_FP64;
-}
-bool stream_enabled_sweep1(int prec) {
-  if (stream_forced() >= 0) return stream_forced() == 1;
-  (void)prec;
-  return true;
-}
-
 int sm_count() {
   static int sms[64] = {};
   int d = 0;
@@ -139,32 +78,6 @@ int sm_count() {
     sms[d] = v;
   }
   return sms[d];
-}
-
-int occupancy_grid(const void *kernel, int threads, size_t smem, int grid) {
-  // blocks of this kernel that fit on an SM at once (registers and shared
-  // memory), cached per kernel, shared memory size and device
-  static std::mutex mu;
-  static std::map<std::tuple<const void *, size_t, int>, int> cache;
-  int d = 0;
-  if (cudaGetDevice(&d) != cudaSuccess) d = 0;
-  int per_sm = 0;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find({kernel, smem, d});
-    if (it != cache.end()) per_sm = it->second;
-  }
-  if (per_sm == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) !=
-            cudaSuccess ||
-        per_sm < 1) {
-      cudaGetLastError();
-      per_sm = 1;
-    }
-    std::lock_guard<std::mutex> lock(mu);
-    cache[{kernel, smem, d}] = per_sm;
-  }
-  return std::max(1, std::min(grid, per_sm * sm_count()));
 }
 
 bool set_smem_attr(const void *kernel, size_t bytes) {
@@ -266,12 +179,14 @@ struct DscaleLaunch {
   const void *d;
   const double *x;
   void *t;
+  int s0, s1;
   cudaStream_t s;
   const int *stop;
-  template <int S, int P>
+  template <int P, int K>
   void run() const {
-    launch(k_sweep_dscale<V, T, S, P>, grid_for_groups(m.nslices, S), kBlock, 0, s, view<V>(m),
-           x, (const V *)d, (T *)t, stop);
+    auto kern = k_sweep_dscale<V, T, P, K>;
+    launch(kern, wave_grid((const void *)kern, (long long)(s1 - s0) * kSlice), kBlock, 0, s,
+           info_view<V>(m), x, (const V *)d, (T *)t, s0, s1, stop);
   }
 };
 
@@ -281,149 +196,17 @@ struct AxpbyLaunch {
   const void *t;
   double alpha, beta;
   double *y;
-  cudaStream_t s;
-  const int *stop;
-  template <int S, int P>
-  void run() const {
-    launch(k_sweep_axpby<V, T, S, P>, grid_for_groups(m.nslices, S), kBlock, 0, s, view<V>(m),
-           (const T *)t, alpha, beta, y, stop);
-  }
-};
-
-template <class V, class T>
-struct DscaleRangeLaunch {
-  const DevSell &m;
-  const void *d;
-  const double *x;
-  void *t;
   int s0, s1;
   cudaStream_t s;
-  template <int S, int P>
-  void run() const {
-    const int g0 = s0 / S, g1 = (s1 + S - 1) / S;
-    k_sweep_dscale_range<V, T, S, P><<<grid_for(g1 - g0), kBlock, 0, s>>>(
-        view<V>(m), x, (const V *)d, (T *)t, g0, g1);
-  }
-};
-
-template <class V, class T>
-struct AxpbyRangeLaunch {
-  const DevSell &m;
-  const void *t;
-  double alpha, beta;
-  double *y;
-  int s0, s1;
-  cudaStream_t s;
-  template <int S, int P>
-  void run() const {
-    const int g0 = s0 / S, g1 = (s1 + S - 1) / S;
-    k_sweep_axpby_range<V, T, S, P><<<grid_for(g1 - g0), kBlock, 0, s>>>(
-        view<V>(m), (const T *)t, alpha, beta, y, g0, g1);
-  }
-};
-
-// The epilogue's row vectors as seen from the host (same rule as row_vecs()).
-template <class V, class T>
-RowVecs host_row_vecs(const EpiDscale<V, T> &e) {
-  return RowVecs{{e.d, nullptr, nullptr}, {(int)sizeof(V), 0, 0}};
-}
-inline RowVecs host_row_vecs(const EpiAxpby &e) {
-  return RowVecs{{e.beta == 0.0 ? nullptr : e.y, nullptr, nullptr}, {8, 0, 0}};
-}
-
-template <class V, class X, class Epi>
-struct StreamLaunch {
-  const DevSell &m;
-  const X *x;
-  Epi epi;
-  int *status;
-  cudaStream_t s;
   const int *stop;
-  int grid;
-  StreamLayout L;
-  size_t smem;
-  bool *launched;
-  template <int S, int P>
+  template <int P, int K>
   void run() const {
-    auto kern = k_stream<V, X, P, Epi>;
-    if (!set_smem_attr((const void *)kern, smem)) return;
-    const int g = occupancy_grid((const void *)kern, kStreamThreads, smem, grid);
-    launch(kern, g, kStreamThreads, smem, s, view<V>(m), (const StageDesc *)m.stages, m.nstages,
-           x, L, epi, status, stop);
-    *launched = true;
+    auto kern = k_sweep_axpby<V, T, P, K>;
+    launch(kern, wave_grid((const void *)kern, (long long)(s1 - s0) * kSlice), kBlock, 0, s,
+           info_view<V>(m), (const T *)t, alpha, beta, y, s0, s1, stop);
   }
 };
 
-// Streaming launch when the layout allows it (returns false otherwise).
-template <class V, class X, class Epi>
-bool try_stream(const DevSell &m, const X *x, const Epi &epi, int *status, cudaStream_t s,
-                const int *stop, bool sweep1 = false) {
-  if (!status || !(sweep1 ? stream_enabled_sweep1(m.prec) : stream_enabled(m.prec)))
-    return false;
-  if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0) return false;  // bulk copies need 16 B
-  const RowVecs rv = host_row_vecs(epi);
-  for (int i = 0; i < kMaxRowVecs; i++)
-    if (rv.p[i] && (reinterpret_cast<uintptr_t>(rv.p[i]) & 15u) != 0) return false;
-  StreamLayout L;
-  size_t smem = 0;
-  const int grid = stream_plan(m, (int)sizeof(X), Epi::kRowVecs, L, smem);
-  if (grid <= 0) return false;
-  bool launched = false;
-  with_pack<V, 1>(m.pack, StreamLaunch<V, X, Epi>{m, x, epi, status, s, stop, grid, L, smem,
-                                                   &launched});
-  return launched;
-}
-
-template <class V, class T>
-void sweep_dscale(const DevSell &m, const void *d, const double *x, void *t, cudaStream_t s,
-                  const int *stop, int *status) {
-  if (try_stream<V>(m, x, EpiDscale<V, T>{(const V *)d, (T *)t}, status, s, stop, true)) return;
-  with_group_pack<V>(group_size(m.prec), m.pack, DscaleLaunch<V, T>{m, d, x, t, s, stop});
-}
-
-template <class V, class T>
-void sweep_axpby(const DevSell &m, const void *t, double alpha, double beta, double *y,
-                 cudaStream_t s, const int *stop, int *status) {
-  if (try_stream<V>(m, (const T *)t, EpiAxpby{alpha, beta, y}, status, s, stop)) return;
-  with_group_pack<V>(group_size(m.prec), m.pack,
-                     AxpbyLaunch<V, T>{m, t, alpha, beta, y, s, stop});
-}
-
-}  // namespace
-
-int launch_sweep_dscale(const DevSell &m, const void *d, const double *x, void *t,
-                        cudaStream_t s, const int *stop, int *status) {
-  if (m.nslices == 0) return AINV_SUCCESS;
-  switch (m.prec) {
-    case AINV_PREC_FP64: sweep_dscale<double, double>(m, d, x, t, s, stop, status); break;
-    case AINV_PREC_FP32: sweep_dscale<float, float>(m, d, x, t, s, stop, status); break;
-    case AINV_PREC_BF16: sweep_dscale<__nv_bfloat16, float>(m, d, x, t, s, stop, status); break;
-    case AINV_PREC_FP32_ACC64: sweep_dscale<f32w, double>(m, d, x, t, s, stop, status); break;
-    case AINV_PREC_BF16_ACC64: sweep_dscale<b16w, double>(m, d, x, t, s, stop, status); break;
-    default:
-      set_error("unknown precision %d", m.prec);
-      return AINV_ERR_ARG;
-  }
-  return check_launch("sweep_dscale");
-}
-
-int launch_sweep_axpby(const DevSell &m, const void *t, double alpha, double beta,
-                       double *y, cudaStream_t s, const int *stop, int *status) {
-  if (m.nslices == 0) return AINV_SUCCESS;
-  switch (m.prec) {
-    case AINV_PREC_FP64: sweep_axpby<double, double>(m, t, alpha, beta, y, s, stop, status); break;
-    case AINV_PREC_FP32: sweep_axpby<float, float>(m, t, alpha, beta, y, s, stop, status); break;
-    case AINV_PREC_BF16: sweep_axpby<__nv_bfloat16, float>(m, t, alpha, beta, y, s, stop, status); break;
-    case AINV_PREC_FP32_ACC64: sweep_axpby<f32w, double>(m, t, alpha, beta, y, s, stop, status); break;
-    case AINV_PREC_BF16_ACC64: sweep_axpby<b16w, double>(m, t, alpha, beta, y, s, stop, status); break;
-    default:
-      set_error("unknown precision %d", m.prec);
-      return AINV_ERR_ARG;
-  }
-  return check_launch("sweep_axpby");
-}
-
-namespace {
 // Storage type V and intermediate type T of a precision, as a tag.
 template <class V_, class T_>
 struct Types {
@@ -446,60 +229,77 @@ int by_prec(int prec, F &&f) {
 }
 
 int check_range(const DevSell &m, int s0, int s1) {
-  if (s0 < 0 || s1 > m.nslices || s0 > s1 || (s0 & 3) != 0) {
+  if (s0 < 0 || s1 > m.nslices || s0 > s1) {
     set_error("slice range [%d, %d) invalid for %d slices", s0, s1, m.nslices);
     return AINV_ERR_ARG;
   }
   return AINV_SUCCESS;
 }
+
+int sweep_dscale(const DevSell &m, const void *d, const double *x, void *t, int s0, int s1,
+                 cudaStream_t s, const int *stop, const char *what) {
+  if (s0 == s1) return AINV_SUCCESS;
+  AINV_TRY(by_prec(m.prec, [&](auto ty) {
+    using Ty = decltype(ty);
+    with_info<typename Ty::V>(
+        m, DscaleLaunch<typename Ty::V, typename Ty::T>{m, d, x, t, s0, s1, s, stop});
+  }));
+  return check_launch(what);
+}
+
+int sweep_axpby(const DevSell &m, const void *t, double alpha, double beta, double *y, int s0,
+                int s1, cudaStream_t s, const int *stop, const char *what) {
+  if (s0 == s1) return AINV_SUCCESS;
+  AINV_TRY(by_prec(m.prec, [&](auto ty) {
+    using Ty = decltype(ty);
+    with_info<typename Ty::V>(m, AxpbyLaunch<typename Ty::V, typename Ty::T>{
+                                     m, t, alpha, beta, y, s0, s1, s, stop});
+  }));
+  return check_launch(what);
+}
+
 }  // namespace
+
+int launch_sweep_dscale(const DevSell &m, const void *d, const double *x, void *t,
+                        cudaStream_t s, const int *stop) {
+  return sweep_dscale(m, d, x, t, 0, m.nslices, s, stop, "sweep_dscale");
+}
+
+int launch_sweep_axpby(const DevSell &m, const void *t, double alpha, double beta,
+                       double *y, cudaStream_t s, const int *stop) {
+  return sweep_axpby(m, t, alpha, beta, y, 0, m.nslices, s, stop, "sweep_axpby");
+}
 
 int launch_sweep_dscale_slices(const DevSell &m, const void *d, const double *x, void *t,
                                int s0, int s1, cudaStream_t s) {
   AINV_TRY(check_range(m, s0, s1));
-  if (s0 == s1) return AINV_SUCCESS;
-  AINV_TRY(by_prec(m.prec, [&](auto ty) {
-    using V = typename decltype(ty)::V;
-    using T = typename decltype(ty)::T;
-    with_group_pack<V>(group_size(m.prec), m.pack, DscaleRangeLaunch<V, T>{m, d, x, t, s0, s1, s});
-  }));
-  return check_launch("sweep_dscale (slices)");
+  return sweep_dscale(m, d, x, t, s0, s1, s, nullptr, "sweep_dscale (slices)");
 }
 
 int launch_sweep_axpby_slices(const DevSell &m, const void *t, double alpha, double beta,
                               double *y, int s0, int s1, cudaStream_t s) {
   AINV_TRY(check_range(m, s0, s1));
-  if (s0 == s1) return AINV_SUCCESS;
-  AINV_TRY(by_prec(m.prec, [&](auto ty) {
-    using V = typename decltype(ty)::V;
-    using T = typename decltype(ty)::T;
-    with_group_pack<V>(group_size(m.prec), m.pack,
-                       AxpbyRangeLaunch<V, T>{m, t, alpha, beta, y, s0, s1, s});
-  }));
-  return check_launch("sweep_axpby (slices)");
+  return sweep_axpby(m, t, alpha, beta, y, s0, s1, s, nullptr, "sweep_axpby (slices)");
 }
 
 int launch_spmv(const DevSell &a, double alpha, const double *x, double beta, double *y,
-                cudaStream_t s, int *status) {
+                cudaStream_t s) {
   if (a.prec != AINV_PREC_FP64) {
     set_error("operator A must be stored in FP64");
     return AINV_ERR_ARG;
   }
-  if (a.nslices == 0) return AINV_SUCCESS;
-  sweep_axpby<double, double>(a, x, alpha, beta, y, s, nullptr, status);
-  return check_launch("spmv");
+  return sweep_axpby(a, x, alpha, beta, y, 0, a.nslices, s, nullptr, "spmv");
 }
 
 int ainv_apply_async(const ainv_handle *h, char trans, double alpha, const double *x,
-                     double beta, double *y, cudaStream_t s, const int *stop, int *status) {
-  int *st = status ? status : h->status;
+                     double beta, double *y, cudaStream_t s, const int *stop) {
   switch (trans) {
     case 'N': case 'n':
-      AINV_TRY(launch_sweep_dscale(h->wt, h->d, x, h->t, s, stop, st));
-      return launch_sweep_axpby(h->z, h->t, alpha, beta, y, s, stop, st);
+      AINV_TRY(launch_sweep_dscale(h->wt, h->d, x, h->t, s, stop));
+      return launch_sweep_axpby(h->z, h->t, alpha, beta, y, s, stop);
     case 'T': case 't': case 'C': case 'c':
-      AINV_TRY(launch_sweep_dscale(h->zt, h->d, x, h->t, s, stop, st));
-      return launch_sweep_axpby(h->w, h->t, alpha, beta, y, s, stop, st);
+      AINV_TRY(launch_sweep_dscale(h->zt, h->d, x, h->t, s, stop));
+      return launch_sweep_axpby(h->w, h->t, alpha, beta, y, s, stop);
     default:
       // psb_err_iarg_invalid_i_ (src/impl/mld_d_base_ainv_solver_apply_vect.f90:64-71)
       set_error("invalid trans '%c'", trans);

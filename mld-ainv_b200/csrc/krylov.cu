@@ -166,15 +166,17 @@ __device__ __forceinline__ bool dots_skip(const KState *st) {
   return st->done != 0;
 }
 
-template <int MODE, int S, int P>
-__global__ void __launch_bounds__(kBlock)
-    k_spmv_dots(SellView<double> m, const double *__restrict__ x, double *__restrict__ y,
+template <int MODE, int P, int K>
+__global__ void __launch_bounds__(kBlock, info_blocks<double, K>())
+    k_spmv_dots(InfoView<double> m, const double *__restrict__ x, double *__restrict__ y,
                 const double *__restrict__ w1, double *__restrict__ w2,
                 const double *__restrict__ w3, const KState *st, SliceOut o) {
   if (dots_skip<MODE>(st)) return;
   SliceSums<dots_of(MODE)> ss{o.sp, o.ld, {}};
-  for_each_row_sliced<S, P>(
-      m, x, [&](int i, double acc) { dots_row<MODE>(i, acc, x, y, w1, w2, w3, ss); },
+  const double *a = dots_operand<MODE>(x, w1);
+  for_each_info<P, K>(
+      m, x, 0, m.nslices, [&](int i) { return a[i]; },
+      [&](int i, double acc, double ai) { dots_row<MODE>(i, acc, ai, y, w2, w3, ss); },
       [&](int s) { ss.end(s); });
 }
 
@@ -186,60 +188,19 @@ __global__ void __launch_bounds__(kBlock)
   for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) r[i] = rtrue[i];
 }
 
-// ---- streaming variants (stream.cuh) ----------------------------------------
-template <int MODE, int P>
-__global__ void __launch_bounds__(kStreamThreads, kStreamMinBlocks)
-    k_stream_dots(SellView<double> m, const StageDesc *__restrict__ stages, int nstages,
-                  StreamLayout L, const double *__restrict__ x, double *__restrict__ y,
-                  const double *__restrict__ w1, double *__restrict__ w2,
-                  const double *__restrict__ w3, KState *st, SliceOut o) {
-  if (dots_skip<MODE>(st)) return;
-  EpiDots<MODE> epi{y, x, w1, w2, w3, {o.sp, o.ld, {}}};
-  stream_rows<P, 1>(m, stages, nstages, x, L, epi, &st->timeout);
-}
-
-// CG sweep 2 with rho = r.z, streaming.
-template <class T>
-struct EpiCgZ {
-  const double *__restrict__ r;
-  double *__restrict__ z;
-  SliceSums<1> ss;
-  static constexpr int kRowVecs = 1;
-  __device__ __host__ __forceinline__ RowVecs row_vecs() const {
-    return RowVecs{{r, nullptr, nullptr}, {8, 0, 0}};
-  }
-  template <class A>
-  __device__ __forceinline__ void post(int i, A acc, const StagedRows &rows) {
-    const double zi = (double)acc;
-    z[i] = zi;
-    ss.v[0] = rows.get<double>(0, i) * zi;
-  }
-  __device__ __forceinline__ void end_slice(int s) { ss.end(s); }
-};
-
-template <class V, class T, int P>
-__global__ void __launch_bounds__(kStreamThreads, kStreamMinBlocks)
-    k_stream_cg_sweep2(SellView<V> m, const StageDesc *__restrict__ stages, int nstages,
-                       StreamLayout L, const T *__restrict__ t, const double *__restrict__ r,
-                       double *__restrict__ z, KState *st, SliceOut o) {
-  if (st->done) return;
-  EpiCgZ<T> epi{r, z, {o.sp, o.ld, {0.0}}};
-  stream_rows<P, stream_rmax<V>()>(m, stages, nstages, t, L, epi, &st->timeout);
-}
-
 // CG: z = Z t (sweep 2 of the AINV apply) fused with rho = r.z.
-template <class V, class T, int S, int P>
-__global__ void __launch_bounds__(kBlock)
-    k_cg_sweep2(SellView<V> m, const T *__restrict__ t, const double *__restrict__ r,
+template <class V, class T, int P, int K>
+__global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
+    k_cg_sweep2(InfoView<V> m, const T *__restrict__ t, const double *__restrict__ r,
                 double *__restrict__ z, const KState *st, SliceOut o) {
   if (st->done) return;
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
-  for_each_row_sliced<S, P>(
-      m, t,
-      [&](int i, auto acc) {
+  for_each_info<P, K>(
+      m, t, 0, m.nslices, [&](int i) { return r[i]; },
+      [&](int i, auto acc, double ri) {
         const double zi = (double)acc;
         z[i] = zi;
-        ss.v[0] = r[i] * zi;
+        ss.v[0] = ri * zi;
       },
       [&](int s) { ss.end(s); });
 }
@@ -342,65 +303,24 @@ struct CgSweep2Launch {
   double *z;
   KState *st;
   SliceOut o;
-  int G;
   cudaStream_t s;
-  template <int S, int P>
+  template <int P, int K>
   void run() const {
-    auto kern = k_cg_sweep2<V, T, S, P>;
-    launch(kern, std::min(G, wave_grid((const void *)kern, m.n)), kBlock, 0, s, view<V>(m),
-           (const T *)t, r, z, st, o);
+    auto kern = k_cg_sweep2<V, T, P, K>;
+    launch(kern, wave_grid((const void *)kern, m.n), kBlock, 0, s, info_view<V>(m), (const T *)t,
+           r, z, st, o);
   }
 };
 
-inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
 template <class V, class T>
-struct StreamCgSweep2Launch {
-  const DevSell &m;
-  StreamLayout L;
-  int grid;
-  size_t smem;
-  const void *t;
-  const double *r;
-  double *z;
-  KState *st;
-  SliceOut o;
-  cudaStream_t s;
-  bool *launched;
-  template <int S, int P>
-  void run() const {
-    auto kern = k_stream_cg_sweep2<V, T, P>;
-    if (!set_smem_attr((const void *)kern, smem)) return;
-    const int g = occupancy_grid((const void *)kern, kStreamThreads, smem, grid);
-    launch(kern, g, kStreamThreads, smem, s, view<V>(m), m.stages, m.nstages, L, (const T *)t, r, z,
-           st, o);
-    *launched = true;
-  }
-};
-
-// Returns true when the streaming kernel ran (its sums are per slice).
-template <class V, class T>
-bool launch_cg_sweep2(const DevSell &m, const void *t, const double *r, double *z,
-                      KState *st, SliceOut o, int G, cudaStream_t s) {
-  if (stream_enabled(m.prec)) {
-    StreamLayout L;
-    size_t smem = 0;
-    const int grid = stream_plan(m, (int)sizeof(T), EpiCgZ<T>::kRowVecs, L, smem);
-    bool launched = false;
-    if (grid > 0 && grid <= G && aligned16(t) && aligned16(r))
-      with_pack<V, 1>(m.pack, StreamCgSweep2Launch<V, T>{m, L, grid, smem, t, r, z, st, o,
-                                                          s, &launched});
-    if (launched) return true;
-  }
-  with_group_pack<V>(group_size(m.prec), m.pack,
-                     CgSweep2Launch<V, T>{m, t, r, z, st, o, G, s});
-  return false;
+void launch_cg_sweep2(const DevSell &m, const void *t, const double *r, double *z, KState *st,
+                      SliceOut o, cudaStream_t s) {
+  with_info<V>(m, CgSweep2Launch<V, T>{m, t, r, z, st, o, s});
 }
 
 template <int MODE>
 struct SpmvDotsLaunch {
-  const SellView<double> &A;
-  int G;
+  const DevSell &A;
   cudaStream_t s;
   const double *x;
   double *y;
@@ -409,63 +329,20 @@ struct SpmvDotsLaunch {
   const double *w3;
   KState *st;
   SliceOut pp;
-  template <int S, int P>
+  template <int P, int K>
   void run() const {
-    auto kern = k_spmv_dots<MODE, S, P>;
-    launch(kern, std::min(G, wave_grid((const void *)kern, A.n)), kBlock, 0, s, A, x, y, w1, w2, w3,
-           st, pp);
+    auto kern = k_spmv_dots<MODE, P, K>;
+    launch(kern, wave_grid((const void *)kern, A.n), kBlock, 0, s, info_view<double>(A), x, y, w1,
+           w2, w3, st, pp);
   }
 };
 
+// y = A x with the dots of MODE.
 template <int MODE>
-struct StreamDotsLaunch {
-  const DevSell &m;
-  StreamLayout L;
-  int grid;
-  size_t smem;
-  cudaStream_t s;
-  const double *x;
-  double *y;
-  const double *w1;
-  double *w2;
-  const double *w3;
-  KState *st;
-  SliceOut pp;
-  bool *launched;
-  template <int S, int P>
-  void run() const {
-    auto kern = k_stream_dots<MODE, P>;
-    if (!set_smem_attr((const void *)kern, smem)) return;
-    const int g = occupancy_grid((const void *)kern, kStreamThreads, smem, grid);
-    launch(kern, g, kStreamThreads, smem, s, view<double>(m), m.stages, m.nstages, L, x, y, w1, w2,
-           w3, st, pp);
-    *launched = true;
-  }
-};
-
-// y = A x with the dots of MODE (streaming when the layout allows; then the
-// sums are per slice and the function returns true).
-template <int MODE>
-bool spmv_dots(const DevSell &Am, int G, cudaStream_t s, const double *x, double *y,
-               const double *w1, double *w2, const double *w3, KState *st, SliceOut pp) {
-  if (stream_enabled(Am.prec)) {
-    StreamLayout L;
-    size_t smem = 0;
-    const int grid = stream_plan(Am, 8, EpiDots<MODE>::kRowVecs, L, smem);
-    const RowVecs rv = EpiDots<MODE>{y, x, w1, w2, w3, {}}.row_vecs();
-    bool launched = false;
-    if (grid > 0 && grid <= G && aligned16(x) && aligned16(rv.p[0]) && aligned16(rv.p[1]) &&
-        aligned16(rv.p[2]))
-      with_pack<double, 1>(Am.pack, StreamDotsLaunch<MODE>{Am, L, grid, smem, s, x, y, w1, w2, w3,
-                                                           st, pp, &launched});
-    if (launched) return true;
-  }
-  const SellView<double> A = view<double>(Am);
-  with_group_pack<double>(group_size(Am.prec), Am.pack,
-                          SpmvDotsLaunch<MODE>{A, G, s, x, y, w1, w2, w3, st, pp});
-  return false;
+void spmv_dots(const DevSell &A, cudaStream_t s, const double *x, double *y, const double *w1,
+               double *w2, const double *w3, KState *st, SliceOut pp) {
+  with_info<double>(A, SpmvDotsLaunch<MODE>{A, s, x, y, w1, w2, w3, st, pp});
 }
-
 
 std::atomic<unsigned long long> g_serial{1};
 
@@ -558,14 +435,14 @@ int get_ws(ainv_csr *a, KrylovWs **out) {
   return AINV_SUCCESS;
 }
 
-bool precond_sweep2_cg(const ainv_handle *h, const double *r, double *z, KState *st,
-                       SliceOut o, int G, cudaStream_t s) {
+void precond_sweep2_cg(const ainv_handle *h, const double *r, double *z, KState *st,
+                       SliceOut o, cudaStream_t s) {
   switch (h->prec) {
-    case AINV_PREC_FP64: return launch_cg_sweep2<double, double>(h->z, h->t, r, z, st, o, G, s);
-    case AINV_PREC_FP32: return launch_cg_sweep2<float, float>(h->z, h->t, r, z, st, o, G, s);
-    case AINV_PREC_FP32_ACC64: return launch_cg_sweep2<f32w, double>(h->z, h->t, r, z, st, o, G, s);
-    case AINV_PREC_BF16_ACC64: return launch_cg_sweep2<b16w, double>(h->z, h->t, r, z, st, o, G, s);
-    default: return launch_cg_sweep2<__nv_bfloat16, float>(h->z, h->t, r, z, st, o, G, s);
+    case AINV_PREC_FP64: return launch_cg_sweep2<double, double>(h->z, h->t, r, z, st, o, s);
+    case AINV_PREC_FP32: return launch_cg_sweep2<float, float>(h->z, h->t, r, z, st, o, s);
+    case AINV_PREC_FP32_ACC64: return launch_cg_sweep2<f32w, double>(h->z, h->t, r, z, st, o, s);
+    case AINV_PREC_BF16_ACC64: return launch_cg_sweep2<b16w, double>(h->z, h->t, r, z, st, o, s);
+    default: return launch_cg_sweep2<__nv_bfloat16, float>(h->z, h->t, r, z, st, o, s);
   }
 }
 
@@ -583,20 +460,20 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
   if (method == AINV_KRYLOV_CG) {
     double *r = w->v(R), *z = w->v(Z), *p = w->v(P), *q = w->v(V), *x = w->v(XW);
     if (h) {
-      AINV_TRY(launch_sweep_dscale(h->wt, h->d, r, h->t, s, stop, &st->timeout));
-      precond_sweep2_cg(h, r, z, st, pp, G, s);
+      AINV_TRY(launch_sweep_dscale(h->wt, h->d, r, h->t, s, stop));
+      precond_sweep2_cg(h, r, z, st, pp, s);
     } else {
       launch(k_cg_ident, std::min(G, wave_grid((const void *)k_cg_ident, n)), kBlock, 0, s, n, r, z,
              st, pp);
     }
     w->fold<1>(FinCgRho{});
     launch(k_cg_p, Gv, kBlock, 0, s, n, z, p, st);
-    spmv_dots<kCgSigma>(A, G, s, p, q, nullptr, nullptr, nullptr, st, pp);
+    spmv_dots<kCgSigma>(A, s, p, q, nullptr, nullptr, nullptr, st, pp);
     w->fold<1>(FinDots<kCgSigma>{nullptr});
     launch(k_cg_xr, std::min(G, wave_grid((const void *)k_cg_xr, n)), kBlock, 0, s, n, p, q, x, r,
            st, pp);
     w->fold<1>(FinCgXr{});
-    spmv_dots<kTrueRes>(A, G, s, x, w->v(RTRUE), w->v(BW), nullptr, r, st, pp);
+    spmv_dots<kTrueRes>(A, s, x, w->v(RTRUE), w->v(BW), nullptr, r, st, pp);
     w->fold<3>(FinDots<kTrueRes>{nullptr});
     launch(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n, w->v(RTRUE), r,
            st);
@@ -605,24 +482,24 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
            *sv = w->v(S), *z = w->v(Z), *t = w->v(T), *x = w->v(XW);
     launch(k_bicg_p, Gv, kBlock, 0, s, n, r, v, p, st);
     if (h) {
-      AINV_TRY(ainv_apply_async(h, 'N', 1.0, p, 0.0, f, s, stop, &st->timeout));
+      AINV_TRY(ainv_apply_async(h, 'N', 1.0, p, 0.0, f, s, stop));
     } else {
       AINV_CUDA_TRY(cudaMemcpyAsync(f, p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     }
-    spmv_dots<kBicgSigma>(A, G, s, f, v, rt, nullptr, nullptr, st, pp);
+    spmv_dots<kBicgSigma>(A, s, f, v, rt, nullptr, nullptr, st, pp);
     w->fold<1>(FinDots<kBicgSigma>{rt});
     launch(k_bicg_s, Gv, kBlock, 0, s, n, r, v, sv, st);
     if (h) {
-      AINV_TRY(ainv_apply_async(h, 'N', 1.0, sv, 0.0, z, s, stop, &st->timeout));
+      AINV_TRY(ainv_apply_async(h, 'N', 1.0, sv, 0.0, z, s, stop));
     } else {
       AINV_CUDA_TRY(cudaMemcpyAsync(z, sv, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     }
-    spmv_dots<kBicgOmega>(A, G, s, z, t, sv, nullptr, nullptr, st, pp);
+    spmv_dots<kBicgOmega>(A, s, z, t, sv, nullptr, nullptr, st, pp);
     w->fold<2>(FinDots<kBicgOmega>{rt});
     launch(k_bicg_xr, std::min(G, wave_grid((const void *)k_bicg_xr, n)), kBlock, 0, s, n, f, z, sv,
            t, rt, x, r, st, pp);
     w->fold<2>(FinBicgXr{});
-    spmv_dots<kTrueRes>(A, G, s, x, w->v(RTRUE), w->v(BW), rt, r, st, pp);
+    spmv_dots<kTrueRes>(A, s, x, w->v(RTRUE), w->v(BW), rt, r, st, pp);
     w->fold<3>(FinDots<kTrueRes>{rt});
     launch(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n, w->v(RTRUE), r,
            st);
@@ -699,7 +576,7 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
          w->out());
   w->fold<1>(FinBnorm{});
   double *rt0 = method == AINV_KRYLOV_BICGSTAB ? w->v(RT) : nullptr;
-  spmv_dots<kInit>(A, w->G, w->s, w->v(XW), w->v(R), w->v(BW), rt0, nullptr, w->st, w->out());
+  spmv_dots<kInit>(A, w->s, w->v(XW), w->v(R), w->v(BW), rt0, nullptr, w->st, w->out());
   w->fold<2>(FinDots<kInit>{rt0});
   AINV_CUDA_TRY(cudaGetLastError());
 

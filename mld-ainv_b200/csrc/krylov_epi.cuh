@@ -33,12 +33,17 @@ constexpr int dots_of(int mode) {
 //               Decides whether r is replaced and whether the convergence
 //               stands; w2 = rt for BiCGSTAB's rho.
 // The row products of the dots go to ss; the fold does the scalar step.
+// a: element i of the vector that every MODE multiplies or subtracts from
+// (dots_operand), which a caller can load before the row sum is known.
+template <int MODE>
+__device__ __forceinline__ const double *dots_operand(const double *x, const double *w1) {
+  return MODE == kCgSigma ? x : w1;
+}
 template <int MODE, class SS>
-__device__ __forceinline__ void dots_row(int i, double acc, const double *__restrict__ x,
-                                         double *__restrict__ y, const double *w1, double *w2,
-                                         const double *w3, SS &ss) {
+__device__ __forceinline__ void dots_row(int i, double acc, double a, double *__restrict__ y,
+                                         double *w2, const double *w3, SS &ss) {
   if constexpr (MODE == kTrueRes || MODE == kInit) {
-    const double ri = w1[i] - acc;
+    const double ri = a - acc;
     y[i] = ri;
     ss.v[0] = ri * ri;
     if constexpr (MODE == kInit) {
@@ -53,11 +58,10 @@ __device__ __forceinline__ void dots_row(int i, double acc, const double *__rest
     }
   } else {
     y[i] = acc;
-    if constexpr (MODE == kCgSigma) ss.v[0] = x[i] * acc;
-    if constexpr (MODE == kBicgSigma) ss.v[0] = w1[i] * acc;
+    if constexpr (MODE == kCgSigma || MODE == kBicgSigma) ss.v[0] = a * acc;
     if constexpr (MODE == kBicgOmega) {
       ss.v[0] = acc * acc;
-      ss.v[1] = acc * w1[i];
+      ss.v[1] = acc * a;
     }
   }
 }

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cstdlib>
+#include <map>
 
 #include "internal.h"
 
@@ -229,6 +230,38 @@ int upload_sell_t(const HostCsr &a, int prec, DevSell &out) {
     iptr[s + 1] = (int)idx.size();
   }
   DevSell m;
+  // slice word groups and the distinct offset lists (padding offsets are 0).
+  // The map is bounded: past kMaxLists distinct lists a new list is appended
+  // without a search, so a matrix whose slices share nothing costs no more
+  // than a copy of its index words.
+  constexpr size_t kMaxLists = 4096;
+  std::vector<int4> info((size_t)ns);
+  std::vector<int> pidx;
+  std::map<std::vector<int>, int> lists;
+  std::vector<int> last;
+  int last_at = -1;
+  for (int s = 0; s < ns; s++) {
+    const int wp = (sptr[s + 1] - sptr[s]) / kSlice;
+    int at = iptr[s];
+    if (om[s]) {
+      const auto b = idx.begin() + iptr[s], e = idx.begin() + iptr[s + 1];
+      if (last_at < 0 || (size_t)wp != last.size() || !std::equal(b, e, last.begin())) {
+        last.assign(b, e);
+        const auto it = lists.find(last);
+        if (it != lists.end()) {
+          last_at = it->second;
+        } else {
+          last_at = (int)pidx.size();
+          pidx.insert(pidx.end(), b, e);
+          pidx.resize((pidx.size() + 3) / 4 * 4, 0);  // 16-byte loads
+          if (lists.size() < kMaxLists) lists.emplace(last, last_at);
+        }
+      }
+      at = last_at;
+    }
+    info[(size_t)s] = make_int4(sptr[s], at, wp, om[s] ? 1 : 0);
+    m.wmax = std::max(m.wmax, wp);
+  }
   m.n = n;
   m.nslices = ns;
   m.nnz = a.nnz();
@@ -308,6 +341,13 @@ int upload_sell_t(const HostCsr &a, int prec, DevSell &out) {
   cudaError_t e = cudaMalloc(&m.sptr, sizeof(int) * sptr.size());
   if (e == cudaSuccess) e = cudaMalloc(&m.iptr, sizeof(int) * iptr.size());
   if (e == cudaSuccess && !idx.empty()) e = cudaMalloc(&m.idx, sizeof(int) * idx.size());
+  if (e == cudaSuccess) e = cudaMalloc(&m.info, sizeof(int4) * info.size());
+  if (e == cudaSuccess)
+    e = cudaMemcpy(m.info, info.data(), sizeof(int4) * info.size(), cudaMemcpyHostToDevice);
+  pidx.resize(pidx.size() + 4, 0);
+  if (e == cudaSuccess) e = cudaMalloc(&m.pidx, sizeof(int) * pidx.size());
+  if (e == cudaSuccess)
+    e = cudaMemcpy(m.pidx, pidx.data(), sizeof(int) * pidx.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !stages.empty())
     e = cudaMalloc(&m.stages, sizeof(StageDesc) * stages.size());
   if (e == cudaSuccess && !stages.empty())
@@ -348,6 +388,8 @@ int upload_sell(const HostCsr &a, int prec, DevSell &out) {
 
 void free_sell(DevSell &m) {
   if (m.stages) cudaFree(m.stages);
+  if (m.info) cudaFree(m.info);
+  if (m.pidx) cudaFree(m.pidx);
   if (m.sptr) cudaFree(m.sptr);
   if (m.iptr) cudaFree(m.iptr);
   if (m.idx) cudaFree(m.idx);

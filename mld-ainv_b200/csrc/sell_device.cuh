@@ -4,6 +4,8 @@
 
 #include <cuda_bf16.h>
 
+#include <climits>
+
 #include <type_traits>
 #include <utility>
 
@@ -245,24 +247,16 @@ constexpr bool pack_ok() {
   return P == 1 || (P * (int)sizeof(V) <= 16 && (P == 2 || P == 4 || P == 8));
 }
 
-// Call f.template run<S, P>() for the runtime S (1, 2, 4) and P.
-template <class V, int S, class F>
+// Call f.template run<P>() for the runtime pack P.
+template <class V, class F>
 inline bool with_pack(int P, const F &f) {
   switch (P) {
-    case 1: f.template run<S, 1>(); return true;
-    case 2: if constexpr (pack_ok<V, 2>()) { f.template run<S, 2>(); return true; } break;
-    case 4: if constexpr (pack_ok<V, 4>()) { f.template run<S, 4>(); return true; } break;
-    case 8: if constexpr (pack_ok<V, 8>()) { f.template run<S, 8>(); return true; } break;
+    case 1: f.template run<1>(); return true;
+    case 2: if constexpr (pack_ok<V, 2>()) { f.template run<2>(); return true; } break;
+    case 4: if constexpr (pack_ok<V, 4>()) { f.template run<4>(); return true; } break;
+    case 8: if constexpr (pack_ok<V, 8>()) { f.template run<8>(); return true; } break;
   }
   return false;
-}
-template <class V, class F>
-inline bool with_group_pack(int S, int P, const F &f) {
-  switch (S) {
-    case 1: return with_pack<V, 1>(P, f);
-    case 4: return with_pack<V, 4>(P, f);
-    default: return with_pack<V, 2>(P, f);
-  }
 }
 
 // Warp-level slice loop: warp w of block b takes slices b*8+w, then every
@@ -415,24 +409,164 @@ __device__ __forceinline__ void group_dot(const SellView<V> &m, const GroupCtx<S
   }
 }
 
-// Visit every row of M: epi(row, acc) for rows < n, S slices per warp step,
-// warps striding over the grid.  [g0, g1) restricts the walk to those groups
-// of S slices (rows stay absolute).
-template <int S, int P, int K = 4, class V, class X, class Epi>
-__device__ __forceinline__ void for_each_row(const SellView<V> &m, const X *__restrict__ x,
-                                             Epi &&epi, int g0 = 0, int g1 = 0x7fffffff) {
-  const int ngroups = min((m.nslices + S - 1) / S, g1);
+// ---- slices through their word groups (DevSell::info) ------------------------
+// A slice's word group gives the address of its values, and of an offset list
+// that many slices share, so one load (prefetched while the previous slice is
+// summed) stands between a warp and all of a slice's values and gathered
+// elements.  The chain slice pointers -> offsets -> gathers of group_dot,
+// three DRAM round trips per step, held the sweeps at 4.5-4.9 TB/s; these
+// run at the copy peak (200^3 FP64: sweep 1 90.3 -> 70.4 us, sweep 2 79.9 ->
+// 60.7 us, 6.4 TB/s each) and beat the bulk-copy pipeline of stream.cuh at
+// every precision and pattern measured (128^3 FP32 40.6 -> 30.8 us per apply,
+// 101^3 BF16 26.8 -> 18.3, 100^3 INVK FP64 83.7 -> 71.4, 128^3 scattered
+// columns FP64 82.3 -> 70.9).
+template <class V>
+struct InfoView {
+  int n, nslices;
+  const int4 *__restrict__ info;
+  const int *__restrict__ pidx;
+  const int *__restrict__ idx;
+  const V *__restrict__ val;
+};
+template <class V>
+inline InfoView<V> info_view(const DevSell &m) {
+  return InfoView<V>{m.n, m.nslices, m.info, m.pidx, m.idx, (const V *)m.val};
+}
+
+// Row `row` of a slice (word group f) dotted with x, K slots at a time.  The
+// gathers of offset-mode slots do not wait for the values: an in-range
+// element is read for zero slots too and replaced by zero, so the products
+// are those of group_slots, in the same order.
+template <int P, int K, class V, class X>
+__device__ __forceinline__ typename Acc<V>::type info_dot(const InfoView<V> &m, const int4 &f,
+                                                          int row, const X *__restrict__ x) {
+  using A = typename Acc<V>::type;
+  static_assert(K % P == 0, "whole packs");
+  constexpr int J = K / P;
   const int lane = threadIdx.x & 31;
-  for (int g = g0 + first_slice(); g < ngroups; g += slice_stride()) {
-    GroupCtx<S> c;
-    group_ctx(m, g, c);
-    typename Acc<V>::type acc[S];
-    group_dot<P, K>(m, c, g, x, acc);
+  const int w = f.z;
+  A acc = A(0);
+  if (f.w) {
+    for (int k0 = 0; k0 < w; k0 += K) {
+      A v[J][P];
+      int c[J][P];
+      X xv[J][P];
 #pragma unroll
-    for (int q = 0; q < S; q++) {
-      const int row = (g * S + q) * kSlice + lane;
-      if (row < m.n) epi(row, acc[q]);
+      for (int j = 0; j < J; j++) {
+        const int k = k0 + j * P;
+        if (k < w) {
+          load_ints<P, false>(m.pidx + f.y + k, c[j]);
+          Pack<V, P>::load(m.val + f.x + (size_t)(k / P) * (kSlice * P) + lane * P, v[j]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < P; e++) {
+            c[j][e] = INT_MIN;  // out of range: not read
+            v[j][e] = A(0);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < J; j++)
+#pragma unroll
+        for (int e = 0; e < P; e++) {
+          const int col = row + c[j][e];
+          xv[j][e] = (unsigned)col < (unsigned)m.n ? __ldg(x + col) : X(0);
+        }
+#pragma unroll
+      for (int j = 0; j < J; j++)
+#pragma unroll
+        for (int e = 0; e < P; e++)
+          acc = madd(v[j][e], v[j][e] != A(0) ? (A)xv[j][e] : A(0), acc);
     }
+  } else {
+    for (int k0 = 0; k0 < w; k0 += K) {
+      A v[J][P];
+      int c[J][P];
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        const int k = k0 + j * P;
+        const size_t pos = (size_t)(k / P) * (kSlice * P) + (size_t)lane * P;
+        if (k < w) {
+          load_ints<P, true>(m.idx + f.y + pos, c[j]);
+          Pack<V, P>::load(m.val + f.x + pos, v[j]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < P; e++) {
+            c[j][e] = INT_MIN;  // out of range: not read
+            v[j][e] = A(0);
+          }
+        }
+      }
+      X xv[J][P];
+#pragma unroll
+      for (int j = 0; j < J; j++)
+#pragma unroll
+        for (int e = 0; e < P; e++)
+          xv[j][e] = (unsigned)c[j][e] < (unsigned)m.n ? __ldg(x + c[j][e]) : X(0);
+#pragma unroll
+      for (int j = 0; j < J; j++)
+#pragma unroll
+        for (int e = 0; e < P; e++)
+          acc = madd(v[j][e], v[j][e] != A(0) ? (A)xv[j][e] : A(0), acc);
+    }
+  }
+  return acc;
+}
+
+// Slots per step (K of info_dot): 4 where every slice has at most 4 (the AINV
+// and INVT factors of the 7-point operators), else 8 (A has 7, INVK(1,1) 23).
+template <int P>
+constexpr int narrow_k() { return P > 4 ? P : 4; }
+// Resident blocks per SM asked for: the loads in flight per thread grow with
+// K and the value size, the warps that hide their latency with the blocks.
+// Narrow steps run best at 6 blocks (40 registers): the 200^3 FP64 apply takes
+// 138, 134, 134 and 173 us at 4, 5, 6 and 8 blocks.  Wide steps need the 64
+// registers of 4 blocks, or spill (100^3 INVK FP64: 71, 76, 86, 84 us), except
+// with 2-byte values (100^3 INVK BF16: 43, 41, 39, 43 us).
+template <class V, int K>
+constexpr int info_blocks() { return K <= 4 || sizeof(V) == 2 ? 6 : 4; }
+
+// Call f.template run<P, K>() for a matrix.
+template <class F>
+struct RunK {
+  const F &f;
+  bool narrow;
+  template <int P>
+  void run() const {
+    if (narrow) f.template run<P, narrow_k<P>()>();
+    else f.template run<P, 8>();
+  }
+};
+template <class V, class F>
+inline bool with_info(const DevSell &m, const F &f) {
+  return with_pack<V>(m.pack, RunK<F>{f, m.wmax <= 4});
+}
+
+// Visit the slices [s0, s1), warps striding over the grid, the next slice's
+// word group loaded while this one is summed: pre(row) starts the epilogue's
+// own loads before the sums, post(row, acc, pre's value) runs for rows < n,
+// and end(s) with the whole warp.
+template <int P, int K, class V, class X, class Pre, class Post, class End>
+__device__ __forceinline__ void for_each_info(const InfoView<V> &m, const X *__restrict__ x,
+                                              int s0, int s1, Pre &&pre, Post &&post,
+                                              End &&end) {
+  const int lane = threadIdx.x & 31;
+  const int step = slice_stride();
+  int s = s0 + first_slice();
+  if (s >= s1) return;
+  int4 f = __ldg(m.info + s);
+  for (;;) {
+    const int sn = s + step;
+    int4 fn = f;
+    if (sn < s1) fn = __ldg(m.info + sn);
+    const int row = s * kSlice + lane;
+    const auto pv = pre(row < m.n ? row : m.n - 1);
+    const auto acc = info_dot<P, K>(m, f, row, x);
+    if (row < m.n) post(row, acc, pv);
+    end(s);
+    if (sn >= s1) break;
+    s = sn;
+    f = fn;
   }
 }
 
@@ -479,31 +613,6 @@ struct SliceSums {
   }
 };
 
-// Visit every slice (warps striding over groups of S slices): epi(row, acc)
-// for each lane whose row is < n, then, with the whole warp, end(slice).
-template <int S, int P, int K = 4, class V, class X, class Epi, class End>
-__device__ __forceinline__ void for_each_row_sliced(const SellView<V> &m,
-                                                    const X *__restrict__ x, Epi &&epi,
-                                                    End &&end) {
-  const int ngroups = (m.nslices + S - 1) / S;
-  const int lane = threadIdx.x & 31;
-  for (int g = first_slice(); g < ngroups; g += slice_stride()) {
-    GroupCtx<S> c;
-    group_ctx(m, g, c);
-    typename Acc<V>::type acc[S];
-    group_dot<P, K>(m, c, g, x, acc);
-#pragma unroll
-    for (int q = 0; q < S; q++) {
-      const int s = g * S + q;
-      if (s < m.nslices) {
-        const int row = s * kSlice + lane;
-        if (row < m.n) epi(row, acc[q]);
-        end(s);
-      }
-    }
-  }
-}
-
 // k<<<g, b, smem, s>>>(args...) through cudaLaunchKernelEx.  (Launching the
 // apply and Krylov kernels with programmatic dependent launch was measured
 // and dropped: the Krylov iteration did not change, and the early-scheduled
@@ -517,15 +626,6 @@ inline void launch(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t s,
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
-}
-
-inline int grid_for(int nslices) { return (nslices + kSlicesPerBlock - 1) / kSlicesPerBlock; }
-
-// Slices per warp step (S of group_dot) for a value type; the default can
-// be overridden with AINV_SLICES_PER_WARP=1|2|4 for tuning.
-int group_size(int prec);
-inline int grid_for_groups(int nslices, int S) {
-  return grid_for((nslices + S - 1) / S);
 }
 
 // Blocks for kernels that end in a grid-wide reduction: at most one resident

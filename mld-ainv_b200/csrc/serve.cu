@@ -690,9 +690,9 @@ __global__ void __launch_bounds__(kBlock, kSrvShareBlocks) k_srv_spmv(const Tabl
                      }))
   SliceSums<dots_of(MODE)> cur{nullptr, 0, {}};
   auto body = [&](int i, int row, double acc) {
-    dots_row<MODE>(row, acc, (const double *)mv.p[i][0], (double *)mv.p[i][1],
-                   (const double *)mv.p[i][2], (double *)mv.p[i][3], (const double *)mv.p[i][4],
-                   cur);
+    const double *w = dots_operand<MODE>((const double *)mv.p[i][0], (const double *)mv.p[i][2]);
+    dots_row<MODE>(row, acc, w[row], (double *)mv.p[i][1], (double *)mv.p[i][3],
+                   (const double *)mv.p[i][4], cur);
   };
   auto end = [&](int i, int s) {
     cur.sp = msp[i];
