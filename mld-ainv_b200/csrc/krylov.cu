@@ -37,6 +37,7 @@
 
 #include "kstate.cuh"
 #include "krylov_epi.cuh"
+#include "persist.cuh"
 
 namespace ainv {
 
@@ -47,6 +48,9 @@ using namespace kstate;
 
 constexpr int kChunk = 8;  // iterations per captured graph launch
 constexpr int kHistCap = 8192;  // iterations whose residual is recorded
+// Arrival counters of the persistent loop, on cache lines of their own.
+constexpr int kBarLine = 32, kBarWords = 3 * kBarLine;
+constexpr int kPersistIters = 1024;  // iterations per launch of it
 
 // Where a reduction kernel stores its sums: dot k of group g (or of slice
 // s, for the streaming kernels) at sp[k*ld + g].
@@ -354,6 +358,7 @@ unsigned long long next_serial() { return g_serial.fetch_add(1); }
 struct KrylovWs {
   int n = 0, G = 0;
   size_t stride = 0;      // doubles between vectors (n rounded up to 32: 256 B aligned)
+  char *mem = nullptr, *hmem = nullptr;  // one device and one page-locked allocation
   double *vec = nullptr;  // 11 vectors of n
   // canonical-order reductions: up to 3 dots' slice sums (ld per dot) and
   // range sums (ldr per dot)
@@ -361,8 +366,12 @@ struct KrylovWs {
   double *sp = nullptr, *rs = nullptr;
   // relative residual per iteration of the last solve (device, host copy)
   double *hist = nullptr;
+  double *hist_h = nullptr;  // page-locked
   std::vector<double> hhist;
   int hcount = 0;
+  // persistent loop: two arrival counters used in turn, and the abort word
+  unsigned *bar = nullptr;
+  unsigned turn = 0;
   KState *st = nullptr;
   KState *hst = nullptr;  // pinned mirror
   cudaStream_t s = nullptr;
@@ -383,12 +392,8 @@ struct KrylovWs {
 void destroy_ws(KrylovWs *w) {
   if (!w) return;
   if (w->exec) cudaGraphExecDestroy(w->exec);
-  if (w->vec) cudaFree(w->vec);
-  if (w->hist) cudaFree(w->hist);
-  if (w->sp) cudaFree(w->sp);
-  if (w->rs) cudaFree(w->rs);
-  if (w->st) cudaFree(w->st);
-  if (w->hst) cudaFreeHost(w->hst);
+  if (w->mem) cudaFree(w->mem);
+  if (w->hmem) cudaFreeHost(w->hmem);
   if (w->ev) cudaEventDestroy(w->ev);
   if (w->s) cudaStreamDestroy(w->s);
   delete w;
@@ -396,7 +401,7 @@ void destroy_ws(KrylovWs *w) {
 
 namespace {
 
-enum { XW = 0, BW, R, RT, P, V, F, S, Z, T, RTRUE, kNumVec };
+enum { XW = 0, BW, R, RT, P, V_, F, S, Z, T_, RTRUE, kNumVec };
 
 int get_ws(ainv_csr *a, KrylovWs **out) {
   if (a->ws) {
@@ -411,20 +416,36 @@ int get_ws(ainv_csr *a, KrylovWs **out) {
   w->n = a->n;
   w->stride = ((size_t)a->n + 31) / 32 * 32;
   w->G = reduction_grid(a->n);
-  cudaError_t e = cudaMalloc(&w->vec, sizeof(double) * kNumVec * w->stride);
   w->ns = (a->n + kSlice - 1) / kSlice;
   w->ld = (w->ns + 31) / 32 * 32;
   w->ng = (w->ns + kGroupSlices - 1) / kGroupSlices;
   w->nr = (w->ng + kFoldRange - 1) / kFoldRange;
   w->ldr = (w->nr + 31) / 32 * 32;
-  if (e == cudaSuccess) e = cudaMalloc(&w->sp, sizeof(double) * 3 * (size_t)w->ld);
-  if (e == cudaSuccess) e = cudaMalloc(&w->rs, sizeof(double) * 3 * (size_t)w->ldr);
-  if (e == cudaSuccess) e = cudaMalloc(&w->hist, sizeof(double) * kHistCap);
-  if (e == cudaSuccess) e = cudaMalloc(&w->st, sizeof(KState));
-  if (e == cudaSuccess) e = cudaMallocHost(&w->hst, sizeof(KState));
+  size_t at = 0;
+  auto part = [&at](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 255) / 256 * 256;
+    return o;
+  };
+  const size_t vec = part(sizeof(double) * kNumVec * w->stride);
+  const size_t sp = part(sizeof(double) * 3 * (size_t)w->ld);
+  const size_t rs = part(sizeof(double) * 3 * (size_t)w->ldr);
+  const size_t hist = part(sizeof(double) * kHistCap);
+  const size_t bar = part(sizeof(unsigned) * kBarWords), st = part(sizeof(KState));
+  cudaError_t e = cudaMalloc(&w->mem, at);
+  if (e == cudaSuccess) e = cudaMemset(w->mem, 0, at);
+  w->vec = reinterpret_cast<double *>(w->mem + vec);
+  w->sp = reinterpret_cast<double *>(w->mem + sp);
+  w->rs = reinterpret_cast<double *>(w->mem + rs);
+  w->hist = reinterpret_cast<double *>(w->mem + hist);
+  w->bar = reinterpret_cast<unsigned *>(w->mem + bar);
+  w->st = reinterpret_cast<KState *>(w->mem + st);
+  const size_t hh = (sizeof(KState) + 255) / 256 * 256;
+  if (e == cudaSuccess) e = cudaMallocHost(&w->hmem, hh + sizeof(double) * kHistCap);
+  w->hst = reinterpret_cast<KState *>(w->hmem);
+  w->hist_h = reinterpret_cast<double *>(w->hmem + hh);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMemset(w->vec, 0, sizeof(double) * kNumVec * w->stride);
   if (e != cudaSuccess) {
     destroy_ws(w);
     set_error("krylov workspace allocation failed: %s", cudaGetErrorString(e));
@@ -458,7 +479,7 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
   cudaStream_t s = w->s;
   const int *stop = &st->done;
   if (method == AINV_KRYLOV_CG) {
-    double *r = w->v(R), *z = w->v(Z), *p = w->v(P), *q = w->v(V), *x = w->v(XW);
+    double *r = w->v(R), *z = w->v(Z), *p = w->v(P), *q = w->v(V_), *x = w->v(XW);
     if (h) {
       AINV_TRY(launch_sweep_dscale(h->wt, h->d, r, h->t, s, stop));
       precond_sweep2_cg(h, r, z, st, pp, s);
@@ -478,8 +499,8 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
     launch(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n, w->v(RTRUE), r,
            st);
   } else {
-    double *r = w->v(R), *rt = w->v(RT), *p = w->v(P), *v = w->v(V), *f = w->v(F),
-           *sv = w->v(S), *z = w->v(Z), *t = w->v(T), *x = w->v(XW);
+    double *r = w->v(R), *rt = w->v(RT), *p = w->v(P), *v = w->v(V_), *f = w->v(F),
+           *sv = w->v(S), *z = w->v(Z), *t = w->v(T_), *x = w->v(XW);
     launch(k_bicg_p, Gv, kBlock, 0, s, n, r, v, p, st);
     if (h) {
       AINV_TRY(ainv_apply_async(h, 'N', 1.0, p, 0.0, f, s, stop));
@@ -548,6 +569,129 @@ int ensure_graph(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int metho
   return AINV_SUCCESS;
 }
 
+// ---- the persistent loop (persist.cuh) -----------------------------------------
+int log2i(int v) {
+  int l = 0;
+  while ((1 << l) < v) l++;
+  return l;
+}
+template <class V>
+PMat<V> pmat(const DevSell &m) {
+  return PMat<V>{info_view<V>(m), log2i(m.pack)};
+}
+
+template <class V, class T, int K, int METHOD, int MB>
+int persist_launch_mb(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b,
+                   double *x, int resume) {
+  PArgs<V, T> p;
+  p.wt = pmat<V>(h->wt);
+  p.z = pmat<V>(h->z);
+  p.a = pmat<double>(a->a);
+  p.d = (const V *)h->d;
+  p.t = (T *)h->t;
+  // CG leaves rt and f free, and BiCGSTAB's check needs no vector of its own
+  // (it uses the p buffer that the next iteration writes)
+  if (METHOD == AINV_KRYLOV_CG)
+    p.w = PVecs{w->v(XW), w->v(BW), {w->v(R), w->v(RT)}, nullptr, {w->v(P), w->v(F)},
+                w->v(V_), nullptr, nullptr, w->v(Z), nullptr};
+  else
+    p.w = PVecs{w->v(XW), w->v(BW), {w->v(R), nullptr}, w->v(RT), {w->v(P), w->v(RTRUE)},
+                w->v(V_), w->v(F), w->v(S), w->v(Z), w->v(T_)};
+  p.xin = x;
+  p.bin = b;
+  p.xout = x;
+  p.gs = w->sp;
+  p.n = w->n;
+  p.ns = w->ns;
+  p.ng = w->ng;
+  p.bar = w->bar + (w->turn & 1u) * kBarLine;
+  p.bar_next = w->bar + ((w->turn + 1) & 1u) * kBarLine;
+  p.abort = reinterpret_cast<int *>(w->bar + 2 * kBarLine);
+  p.st = w->st;
+  p.resume = resume;
+  p.max_iters = kPersistIters;
+  auto kern = k_persist<V, T, K, METHOD, MB>;
+  static const int per_sm = [&] {
+    int v = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, kPBlock, 0) != cudaSuccess) v = 0;
+    cudaGetLastError();
+    return v;
+  }();
+  if (per_sm < 1) return AINV_ERR_UNSUPPORTED;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = std::min((w->ng + kPTeams - 1) / kPTeams,
+                         std::min(per_sm, MB) * sm_count());
+  cfg.blockDim = kPBlock;
+  cfg.stream = w->s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) {
+    cudaGetLastError();
+    return AINV_ERR_UNSUPPORTED;
+  }
+  w->turn++;
+  return AINV_SUCCESS;
+}
+
+template <class V, class T, int K, int METHOD>
+int persist_launch(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b,
+                   double *x, int resume) {
+  return w->ng <= kPTeams * sm_count()
+             ? persist_launch_mb<V, T, K, METHOD, 1>(w, h, a, b, x, resume)
+             : persist_launch_mb<V, T, K, METHOD, 2>(w, h, a, b, x, resume);
+}
+
+template <int K, int METHOD>
+int persist_prec(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b, double *x,
+                 int resume) {
+  switch (h->prec) {
+    case AINV_PREC_FP64: return persist_launch<double, double, K, METHOD>(w, h, a, b, x, resume);
+    case AINV_PREC_FP32: return persist_launch<float, float, K, METHOD>(w, h, a, b, x, resume);
+    case AINV_PREC_FP32_ACC64: return persist_launch<f32w, double, K, METHOD>(w, h, a, b, x, resume);
+    case AINV_PREC_BF16_ACC64: return persist_launch<b16w, double, K, METHOD>(w, h, a, b, x, resume);
+    default: return persist_launch<__nv_bfloat16, float, K, METHOD>(w, h, a, b, x, resume);
+  }
+}
+
+int persist(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b, double *x,
+            int method, int resume) {
+  const bool narrow = h->wt.wmax <= 4 && h->z.wmax <= 4;
+  if (method == AINV_KRYLOV_CG)
+    return narrow ? persist_prec<4, AINV_KRYLOV_CG>(w, h, a, b, x, resume)
+                  : persist_prec<8, AINV_KRYLOV_CG>(w, h, a, b, x, resume);
+  return narrow ? persist_prec<4, AINV_KRYLOV_BICGSTAB>(w, h, a, b, x, resume)
+                : persist_prec<8, AINV_KRYLOV_BICGSTAB>(w, h, a, b, x, resume);
+}
+
+// What a finished solve reports (state and residuals are in page-locked memory).
+int finish_solve(KrylovWs *w, int itmax, int *iter, double *err) {
+  const KState &f = *w->hst;
+  w->last = f;
+  w->hcount = std::min(std::max(f.iter, 0), kHistCap);
+  w->hhist.assign(w->hist_h, w->hist_h + w->hcount);
+  if (iter) *iter = f.iter;
+  if (err) *err = sqrt(f.rn2) / f.bn2;
+  if (f.timeout) {
+    set_error("a device wait of the Krylov loop ran past its time limit");
+    return AINV_ERR_TIMEOUT;
+  }
+  if (!f.done) {
+    set_error("krylov loop did not terminate");
+    return AINV_ERR_INTERNAL;
+  }
+  if (f.status != AINV_SUCCESS) {
+    switch (f.status) {
+      case AINV_ERR_NOCONV: set_error("itmax (%d) reached, err %.3e", itmax, sqrt(f.rn2) / f.bn2); break;
+      case AINV_ERR_BREAKDOWN: set_error("Krylov breakdown at iteration %d", f.iter); break;
+      default: set_error("non-finite residual at iteration %d", f.iter); break;
+    }
+  }
+  return f.status;
+}
+
 }  // namespace
 
 int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, int method,
@@ -560,8 +704,6 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   // order after the caller's stream
   AINV_CUDA_TRY(cudaEventRecord(w->ev, user));
   AINV_CUDA_TRY(cudaStreamWaitEvent(w->s, w->ev, 0));
-  AINV_CUDA_TRY(cudaMemcpyAsync(w->v(XW), x, bytes, cudaMemcpyDeviceToDevice, w->s));
-  AINV_CUDA_TRY(cudaMemcpyAsync(w->v(BW), b, bytes, cudaMemcpyDeviceToDevice, w->s));
   KState init{};
   init.eps = eps;
   init.itmax = itmax;
@@ -571,6 +713,29 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   init.hist_cap = kHistCap;
   *w->hst = init;
   AINV_CUDA_TRY(cudaMemcpyAsync(w->st, w->hst, sizeof(KState), cudaMemcpyHostToDevice, w->s));
+  const bool persistent =
+      h && n <= kPMaxRows && w->ng <= kPMaxPerTeam * kPTeams * 2 * sm_count();
+  if (persistent) {
+    for (int resume = 0;; resume = 1) {
+      const int rc = persist(w, h, a, b, x, method, resume);
+      if (rc == AINV_ERR_UNSUPPORTED && !resume) break;  // no cooperative launch: plain loop
+      AINV_TRY(rc);
+      AINV_CUDA_TRY(cudaMemcpyAsync(w->hst, w->st, sizeof(KState), cudaMemcpyDeviceToHost, w->s));
+      AINV_CUDA_TRY(cudaMemcpyAsync(w->hist_h, w->hist,
+                                    sizeof(double) * (size_t)std::min(itmax, kHistCap),
+                                    cudaMemcpyDeviceToHost, w->s));
+      AINV_CUDA_TRY(cudaStreamSynchronize(w->s));
+      if (w->hst->timeout)
+        AINV_CUDA_TRY(cudaMemset(w->bar, 0, sizeof(unsigned) * kBarWords));
+      if (w->hst->done || w->hst->timeout) {
+        AINV_CUDA_TRY(cudaEventRecord(w->ev, w->s));
+        AINV_CUDA_TRY(cudaStreamWaitEvent(user, w->ev, 0));
+        return finish_solve(w, itmax, iter, err);
+      }
+    }
+  }
+  AINV_CUDA_TRY(cudaMemcpyAsync(w->v(XW), x, bytes, cudaMemcpyDeviceToDevice, w->s));
+  AINV_CUDA_TRY(cudaMemcpyAsync(w->v(BW), b, bytes, cudaMemcpyDeviceToDevice, w->s));
   const DevSell &A = a->a;
   launch(k_bnorm, std::min(w->G, wave_grid((const void *)k_bnorm, n)), kBlock, 0, w->s, n, w->v(BW),
          w->out());
@@ -597,34 +762,13 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   }
   AINV_CUDA_TRY(cudaMemcpyAsync(x, w->v(XW), bytes, cudaMemcpyDeviceToDevice, w->s));
   AINV_CUDA_TRY(cudaMemcpyAsync(w->hst, w->st, sizeof(KState), cudaMemcpyDeviceToHost, w->s));
+  AINV_CUDA_TRY(cudaMemcpyAsync(w->hist_h, w->hist,
+                                sizeof(double) * (size_t)std::min(itmax, kHistCap),
+                                cudaMemcpyDeviceToHost, w->s));
   AINV_CUDA_TRY(cudaStreamSynchronize(w->s));
   AINV_CUDA_TRY(cudaEventRecord(w->ev, w->s));
   AINV_CUDA_TRY(cudaStreamWaitEvent(user, w->ev, 0));
-  const KState &f = *w->hst;
-  w->last = f;
-  w->hcount = std::min(std::max(f.iter, 0), kHistCap);
-  w->hhist.resize((size_t)w->hcount);
-  if (w->hcount > 0)
-    AINV_CUDA_TRY(cudaMemcpy(w->hhist.data(), w->hist, sizeof(double) * (size_t)w->hcount,
-                             cudaMemcpyDeviceToHost));
-  if (iter) *iter = f.iter;
-  if (err) *err = sqrt(f.rn2) / f.bn2;
-  if (f.timeout) {
-    set_error("a device wait of the Krylov loop ran past its time limit");
-    return AINV_ERR_TIMEOUT;
-  }
-  if (!f.done) {
-    set_error("krylov loop did not terminate");
-    return AINV_ERR_INTERNAL;
-  }
-  if (f.status != AINV_SUCCESS) {
-    switch (f.status) {
-      case AINV_ERR_NOCONV: set_error("itmax (%d) reached, err %.3e", itmax, sqrt(f.rn2) / f.bn2); break;
-      case AINV_ERR_BREAKDOWN: set_error("Krylov breakdown at iteration %d", f.iter); break;
-      default: set_error("non-finite residual at iteration %d", f.iter); break;
-    }
-  }
-  return f.status;
+  return finish_solve(w, itmax, iter, err);
 }
 
 }  // namespace ainv

@@ -1,0 +1,690 @@
+// The Krylov loops as one persistent kernel.
+//
+// Below about half a million rows an iteration is bound by its launches, not
+// by its bytes: at 40^3 a CG iteration was 11 launches of 2.3-5.5 us (34 us)
+// for 1.7 us of L2 traffic, a BiCGSTAB iteration 20 (52 us).  As phases of
+// one kernel they take 11.2 and 20.8 us: per phase about 0.8 us from the
+// first gather to the group sums, 1.0 us at the barrier and, where a dot is
+// folded, 1.2 us.  Here the blocks of one cooperative grid run whole
+// iterations, with a grid barrier where one phase reads what another block
+// wrote in the phase before:
+//
+//   CG        z = Z t, rho | p = z + beta p, q = A p, sigma |
+//             x += alpha p, r -= alpha q, ||r||, t = D^-1 W^T r |
+//   BiCGSTAB  p = r + beta (p - omega v), t = D^-1 W^T p | f = Z t |
+//             v = A f, sigma | s = r - alpha v, t = D^-1 W^T s | z = Z t |
+//             t' = A z, omega | x += alpha f + omega z, r = s - omega t',
+//             ||r||, rho |
+//
+// A vector update feeds the product that follows it without a barrier in
+// between: the product forms the updated element of every column it gathers
+// (the same two roundings that the row's owner stores), so p, s and CG's r
+// are never gathered from memory in the phase that writes them (p and CG's
+// r alternate between two buffers).
+//
+// Sums keep the canonical order (sell_device.cuh).  A team of 8 warps takes
+// the 8 slices of a group together and stores the group's sum; after the
+// barrier every block folds all group sums itself and performs the scalar
+// step on its own copy of the state, so a reduction costs no second barrier.
+// Iterates are therefore those of the multi-kernel loop, bit for bit.
+//
+// Matrix words do not change during the loop.  Up to one group per team the
+// blocks run one per SM with 128 registers, and a warp keeps its slices of
+// the three matrices in them (12.4 -> 11.2 us per CG iteration at 40^3);
+// above that, two blocks per SM with 64 registers read them in each phase.
+//
+// Every wait is bounded (kWaitNs); a block that gives up sets the abort word,
+// which ends the others' waits, and the state's timeout flag.
+#pragma once
+
+#include "krylov_epi.cuh"
+
+namespace ainv {
+namespace dev {
+
+constexpr int kPTeams = 2;  // groups per block and step
+constexpr int kPBufs = 4;   // group-sum buffers used in turn
+constexpr int kPBlock = kPTeams * kFoldThreads;
+constexpr int kPWarps = kPBlock / 32;
+// Groups per team up to which a solve runs here.  Past it a phase is bound by
+// the bytes it moves, and the plain kernels, with 48 warps per SM against 32
+// and wide loads, move them faster: us per iteration here / there at 52^3 CG
+// 16.3 / 33, 64^3 CG 23.9 / 38, 64^3 BiCGSTAB 42.5 / 57 (2 groups), 80^3 CG
+// 42 / 45, 80^3 BiCGSTAB 77 / 73 (4 groups), 100^3 BiCGSTAB 139 / 120.
+constexpr int kPMaxPerTeam = 3;
+// Ranges a block folds in one step (one lane each): 32 ranges of 256 groups.
+constexpr int kPMaxRanges = 32;
+constexpr long long kPMaxRows = (long long)kPMaxRanges * kFoldRange * kGroupSlices * kSlice;
+
+template <class V>
+struct PMat {
+  InfoView<V> m;
+  int lg;  // log2 of the pack
+};
+
+// The vectors of a loop.  r and p alternate: iteration k reads [k & 1] and
+// writes [(k + 1) & 1] (BiCGSTAB keeps r in r[0]).
+struct PVecs {
+  double *x, *b, *r[2], *rt, *p[2], *v, *f, *s, *z, *t;
+};
+
+template <class V, class T>
+struct PArgs {
+  PMat<V> wt, z;
+  PMat<double> a;
+  const V *d;
+  T *t;  // apply intermediate
+  PVecs w;
+  const double *xin, *bin;  // start: x0 and b (first launch of a solve)
+  double *xout;             // the solution goes here when the loop ends
+  double *gs;               // group sums: kPBufs buffers of 3 x ng
+  int n, ns, ng;
+  unsigned *bar, *bar_next;  // this launch's arrival counter; the next one's, cleared here
+  int *abort;
+  KState *st;
+  int resume;     // continue from *st
+  int max_iters;  // iterations of this launch at most
+};
+
+struct PShared {
+  KState k;
+  double tree[3][kPMaxRanges * 8];
+  double slice[kPTeams][2][3][kGroupSlices];
+  double rho;
+  int dead;
+};
+
+__device__ __forceinline__ void team_sync(int team) {
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kFoldThreads) : "memory");
+}
+__device__ __forceinline__ void red_release(unsigned *p, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Arrivals of nb blocks at a counter that only grows.
+struct GridBarrier {
+  unsigned *ctr;
+  int *abort;
+  unsigned nb, target;
+  // Called by every thread of the block; false once a wait was given up
+  // (by any block).
+  __device__ __forceinline__ bool wait(PShared &sh) {
+    // The block's writes reach the other blocks by the release of thread 0
+    // (the block barrier orders them before it), theirs this block by its
+    // acquire.
+    __syncthreads();
+    target += nb;
+    if (threadIdx.x == 0 && nb > 1) {
+      red_release(ctr, 1u);
+      if (ld_acquire(ctr) < target) {
+        const unsigned long long t0 = global_ns();
+        for (unsigned it = 1;; ++it) {
+          if (ld_acquire(ctr) >= target) break;
+          if ((it & 63u) == 0 &&
+              (*(volatile int *)abort != 0 || global_ns() - t0 > kWaitNs || it > (1u << 30))) {
+            *(volatile int *)abort = 1;
+            sh.dead = 1;
+            break;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    return sh.dead == 0;
+  }
+};
+
+// ---- a slice's static words ------------------------------------------------
+// The first K slots of the lane's row: values and columns (-1: not read).
+template <class V, int K>
+struct Slab {
+  typename Acc<V>::type v[K];
+  int c[K];
+  int4 f;
+};
+
+__device__ __forceinline__ double ldk(const double *p) { return __ldg(p); }
+template <class V>
+__device__ __forceinline__ typename Acc<V>::type ldk(const V *p) { return ldd(p); }
+
+template <int K, class V>
+__device__ __forceinline__ void slab_slots(const PMat<V> &a, const int4 &f, int row, int k0,
+                                           typename Acc<V>::type (&v)[K], int (&c)[K]) {
+  using A = typename Acc<V>::type;
+  const int lane = threadIdx.x & 31;
+  const int pm = (1 << a.lg) - 1;
+#pragma unroll
+  for (int j = 0; j < K; j++) {
+    const int k = k0 + j;
+    if (k < f.z) {
+      const int pos = ((k >> a.lg) << (5 + a.lg)) + (lane << a.lg) + (k & pm);
+      v[j] = ldk(a.m.val + f.x + pos);
+      c[j] = f.w ? row + __ldg(a.m.pidx + f.y + k) : __ldg(a.m.idx + f.y + pos);
+      if ((unsigned)c[j] >= (unsigned)a.m.n) c[j] = -1;
+    } else {
+      v[j] = A(0);
+      c[j] = -1;
+    }
+  }
+}
+
+template <class V>
+__device__ __forceinline__ int4 slice_info(const PMat<V> &a, int s) {
+  return s < a.m.nslices ? __ldg(a.m.info + s) : make_int4(0, 0, 0, 1);
+}
+template <int K, class V>
+__device__ __forceinline__ void slab_load(const PMat<V> &a, const int4 &f, int row,
+                                          Slab<V, K> &b) {
+  b.f = f;
+  slab_slots<K>(a, f, row, 0, b.v, b.c);
+}
+
+// The lane's row dotted with the gathered vector g (g(column) gives an
+// element), G::kBatch gathers in flight; slots in order, zero slots add 0.
+template <class G, int K, class A>
+__device__ __forceinline__ void slab_sum(const A (&v)[K], const int (&c)[K], const G &g, A &acc) {
+  constexpr int B = G::kBatch < K ? G::kBatch : K;
+#pragma unroll
+  for (int j0 = 0; j0 < K; j0 += B) {
+    A xv[B];
+#pragma unroll
+    for (int j = 0; j < B; j++) xv[j] = c[j0 + j] >= 0 ? (A)g(c[j0 + j]) : A(0);
+#pragma unroll
+    for (int j = 0; j < B; j++)
+      acc = madd(v[j0 + j], v[j0 + j] != A(0) ? xv[j] : A(0), acc);
+  }
+}
+
+template <int K, class V, class G>
+__device__ __forceinline__ typename Acc<V>::type slab_dot(const PMat<V> &a, const Slab<V, K> &b,
+                                                          int row, const G &g) {
+  using A = typename Acc<V>::type;
+  A acc = A(0);
+  slab_sum(b.v, b.c, g, acc);
+  for (int k0 = K; k0 < b.f.z; k0 += K) {
+    A v[K];
+    int c[K];
+    slab_slots<K>(a, b.f, row, k0, v, c);
+    slab_sum(v, c, g, acc);
+  }
+  return acc;
+}
+
+// ---- gathered vectors ---------------------------------------------------------
+// Loads are coherent at the barriers (not the read-only path): these vectors
+// are written while the kernel runs.
+template <class X>
+struct GVec {
+  static constexpr int kBatch = 8;
+  const X *x;
+  __device__ __forceinline__ X operator()(int c) const { return __ldca(x + c); }
+};
+// CG: p = z (first iteration) or z + beta p.
+template <int B>
+struct GCgP {
+  static constexpr int kBatch = B;
+  const double *z, *p;
+  double beta;
+  bool first;
+  __device__ __forceinline__ double operator()(int c) const {
+    const double zc = __ldca(z + c);
+    return first ? zc : zc + beta * __ldca(p + c);
+  }
+};
+// r - alpha q (CG's r, BiCGSTAB's s).
+template <int B>
+struct GSub {
+  static constexpr int kBatch = B;
+  const double *r, *q;
+  double alpha;
+  __device__ __forceinline__ double operator()(int c) const {
+    return __ldca(r + c) - alpha * __ldca(q + c);
+  }
+};
+// BiCGSTAB: p = r (first iteration) or r + beta (p - omega v).
+template <int B>
+struct GBiP {
+  static constexpr int kBatch = B;
+  const double *r, *p, *v;
+  double beta, omega;
+  bool first;
+  __device__ __forceinline__ double operator()(int c) const {
+    const double rc = __ldca(r + c);
+    return first ? rc : rc + beta * (__ldca(p + c) - omega * __ldca(v + c));
+  }
+};
+
+// ---- phases ---------------------------------------------------------------------
+// Blocks lb of nb walk the groups, a team per group, a warp per slice:
+// body(s, row, v) with the warp's slice and the lane's row (which may be past
+// n), then, for NV > 0, the group sums of v[0..NV) go to gs.
+template <int NV, class Body>
+__device__ __forceinline__ void for_groups(int n, int ns, int ng, int lb, int nb, PShared &sh,
+                                           double *gs, Body &&body) {
+  const int team = threadIdx.x / kFoldThreads, lane = threadIdx.x & 31;
+  const int warp = (threadIdx.x / 32) % kGroupSlices;
+  int buf = 0;
+  for (int g = lb * kPTeams + team; g < ng; g += nb * kPTeams) {
+    const int s = g * kGroupSlices + warp;
+    double v[NV > 0 ? NV : 1] = {};
+    if (s < ns) body(s, s * kSlice + lane, v);
+    if constexpr (NV > 0) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const double w = warp_tree(v[k]);
+        if (lane == 0) sh.slice[team][buf][k][warp] = w;
+      }
+      team_sync(team);
+      const int t = threadIdx.x % kFoldThreads;
+      if (t < NV) {
+        double sum = 0.0;
+#pragma unroll
+        for (int j = 0; j < kGroupSlices; j++)
+          if (g * kGroupSlices + j < ns) sum = __dadd_rn(sum, sh.slice[team][buf][t][j]);
+        gs[(size_t)t * ng + g] = sum;
+      }
+      buf ^= 1;
+    }
+  }
+}
+
+// Every block folds the group sums (steps 3 and 4 of the canonical order;
+// at most kPMaxRanges ranges) and runs fin on its copy of the state.
+// dot k's group sums are at src[k].
+template <int NV, class Fin>
+__device__ __forceinline__ void fold_groups(const double *const (&src)[NV], int ng, PShared &sh,
+                                            Fin &&fin) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int nt = (ng + 31) / 32;  // warp trees with groups
+  for (int u0 = warp; u0 < nt; u0 += 4 * kPWarps) {
+    double v[4][NV];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int g = (u0 + q * kPWarps) * 32 + lane;
+#pragma unroll
+      for (int k = 0; k < NV; k++) v[q][k] = g < ng ? __ldcg(src[k] + g) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int u = u0 + q * kPWarps;
+      if (u < nt) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+          const double t = warp_tree(__dadd_rn(0.0, v[q][k]));
+          if (lane == 0) sh.tree[k][u] = t;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double tot[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      double r = 0.0;
+#pragma unroll
+      for (int w = 0; w < 8; w++)
+        if (lane * 8 + w < nt) r = __dadd_rn(r, sh.tree[k][lane * 8 + w]);
+      r = __dadd_rn(0.0, r);
+      // one range: the tree over the ranges would add zeros to it
+      if (nt > 8) r = warp_tree(r);
+      tot[k] = __dadd_rn(0.0, r);
+    }
+    if (lane == 0) fin(tot);
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ bool periodic_check(const KState &k) {
+  return !k.done && k.check_every > 0 && k.iter > 0 && k.iter % k.check_every == 0;
+}
+
+template <class V, class T, int K, int METHOD, int MB>
+struct PLoop {
+  static constexpr int KA = 8;  // slots of A per step
+  static constexpr bool kKeep = MB == 1 && K <= 4;
+  static constexpr int kB = MB == 1 ? 8 : 4;  // formed elements in flight
+  const PArgs<V, T> &a;
+  PShared &sh;
+  GridBarrier bar;
+  int lb, nb;
+  Slab<V, K> hw, hz;    // the warp's first slice of W^T, Z
+  Slab<double, KA> ha;  // and of A
+  int par = 0;     // group-sum buffer
+
+  __device__ __forceinline__ PLoop(const PArgs<V, T> &args, PShared &shared, int lb_, int nb_)
+      : a(args), sh(shared), bar{args.bar, args.abort, (unsigned)nb_, 0u}, lb(lb_), nb(nb_) {
+    const int team = threadIdx.x / kFoldThreads;
+    const int s0 =
+        (lb * kPTeams + team) * kGroupSlices + (int)(threadIdx.x / 32) % kGroupSlices;
+    const int row = s0 * kSlice + (int)(threadIdx.x & 31);
+    hw.f = slice_info(a.wt, s0);
+    hz.f = slice_info(a.z, s0);
+    ha.f = slice_info(a.a, s0);
+    if constexpr (kKeep) {
+      slab_load<K>(a.wt, hw.f, row, hw);
+      slab_load<K>(a.z, hz.f, row, hz);
+      slab_load<KA>(a.a, ha.f, row, ha);
+    }
+  }
+  __device__ __forceinline__ double *gs() const { return a.gs + (size_t)par * 3 * a.ng; }
+  __device__ __forceinline__ void next_buf() { par = (par + 1) % kPBufs; }
+  template <int NV, class Fin>
+  __device__ __forceinline__ void fold_at(const double *sums, Fin &&fin) {
+    const double *src[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) src[k] = sums + (size_t)k * a.ng;
+    fold_groups<NV>(src, a.ng, sh, fin);
+  }
+  __device__ __forceinline__ bool sync() { return bar.wait(sh); }
+  template <int NV, class Body>
+  __device__ __forceinline__ void groups(Body &&body) {
+    for_groups<NV>(a.n, a.ns, a.ng, lb, nb, sh, gs(), body);
+  }
+  template <int NV, class Fin>
+  __device__ __forceinline__ void fold(Fin &&fin) {
+    fold_at<NV>(gs(), fin);
+    next_buf();
+  }
+
+  // Row `row` (of a row past the end, the last one: its loads are in bounds).
+  __device__ __forceinline__ int clamp(int row) const { return row < a.n ? row : a.n - 1; }
+
+  // body(row, slab, v) for the warp's slice of every group.  The first slice
+  // (h) is kept in registers through the loop where they suffice (kKeep:
+  // most systems have one group per team there), else its word group is;
+  // the next slice's word group is loaded while this slice is summed.
+  template <int NV, int KK, class U, class Body>
+  __device__ __forceinline__ void slabs(const PMat<U> &m, const Slab<U, KK> &h, Body &&body) {
+    int4 f = h.f;
+    bool head = true;
+    groups<NV>([&](int s, int row, auto &v) {
+      const int4 fn = slice_info(m, s + nb * kPTeams * kGroupSlices);
+      if (kKeep && head) {
+        body(row, h, v);
+      } else {
+        Slab<U, KK> b;
+        slab_load<KK>(m, f, row, b);
+        body(row, b, v);
+      }
+      head = false;
+      f = fn;
+    });
+  }
+
+  // In each of the three, pre(row) loads what the row's owner needs besides
+  // the gathers, so that both are in flight together, and post stores.
+  // t = D^-1 W^T g.
+  template <int NV, class G, class Pre, class Post>
+  __device__ __forceinline__ void sweep1(const G &g, Pre &&pre, Post &&post) {
+    slabs<NV, K>(a.wt, hw, [&](int row, const Slab<V, K> &b, auto &v) {
+      const auto o = pre(clamp(row));
+      const auto d = ldk(a.d + clamp(row));
+      const auto acc = slab_dot<K>(a.wt, b, row, g);
+      if (row < a.n) {
+        a.t[row] = (T)(d * acc);
+        post(row, o, v);
+      }
+    });
+  }
+  // dst = Z t.
+  template <int NV, class Pre, class Post>
+  __device__ __forceinline__ void sweep2(double *dst, Pre &&pre, Post &&post) {
+    const GVec<T> g{a.t};
+    slabs<NV, K>(a.z, hz, [&](int row, const Slab<V, K> &b, auto &v) {
+      const auto o = pre(clamp(row));
+      const auto acc = slab_dot<K>(a.z, b, row, g);
+      if (row < a.n) {
+        const double z = (double)acc;
+        dst[row] = z;
+        post(row, z, o, v);
+      }
+    });
+  }
+  // (A g)[row] for post.
+  template <int NV, class G, class Pre, class Post>
+  __device__ __forceinline__ void product(const G &g, Pre &&pre, Post &&post) {
+    slabs<NV, KA>(a.a, ha, [&](int row, const Slab<double, KA> &b, auto &v) {
+      const auto o = pre(clamp(row));
+      const double acc = slab_dot<KA>(a.a, b, row, g);
+      if (row < a.n) post(row, acc, o, v);
+    });
+  }
+
+  // x = x0, b, r = b - A x0 (and rt = r), ||b||, ||r||.
+  __device__ __forceinline__ bool init() {
+    product<2>(
+        GVec<double>{a.xin}, [&](int i) { return make_double2(a.bin[i], a.xin[i]); },
+        [&](int i, double acc, double2 o, double (&v)[2]) {
+          const double r = o.x - acc;
+          a.w.x[i] = o.y;
+          a.w.b[i] = o.x;
+          a.w.r[0][i] = r;
+          if (METHOD == AINV_KRYLOV_BICGSTAB) a.w.rt[i] = r;
+          v[0] = o.x * o.x;
+          v[1] = r * r;
+        });
+    if (!sync()) return false;
+    fold<2>([&](const double (&v)[2]) {
+      const double bn = sqrt(v[0]);
+      sh.k.bn2 = (bn == 0.0) ? 1.0 : bn;
+      const double pr[3] = {v[1], METHOD == AINV_KRYLOV_BICGSTAB ? v[1] : 0.0, 0.0};
+      kstate::finish_dots<kInit>(&sh.k, pr, false, nullptr);
+    });
+    return true;
+  }
+
+  // The true-residual check at the end of an iteration (r: the current
+  // residual, scratch: a dead vector).  *replaced: r changed (a barrier
+  // follows the change).
+  __device__ __forceinline__ bool check(double *r, double *scratch, bool *replaced) {
+    *replaced = false;
+    const KState &k = sh.k;
+    const bool verify = k.done && k.status == AINV_SUCCESS && !k.verified;
+    if (!verify && !periodic_check(k)) return true;
+    const double *rt = METHOD == AINV_KRYLOV_BICGSTAB ? a.w.rt : nullptr;
+    product<3>(
+        GVec<double>{a.w.x}, [&](int i) { return make_double2(a.w.b[i], r[i]); },
+        [&](int i, double acc, double2 o, double (&v)[3]) {
+          const double ri = o.x - acc, g = ri - o.y;
+          scratch[i] = ri;
+          v[0] = ri * ri;
+          v[1] = g * g;
+          if (rt) v[2] = rt[i] * ri;
+        });
+    if (!sync()) return false;
+    fold<3>([&](const double (&v)[3]) {
+      kstate::finish_dots<kTrueRes>(&sh.k, v, verify, rt);
+    });
+    if (k.replace) {
+      groups<0>([&](int, int row, auto &) {
+        if (row < a.n) r[row] = scratch[row];
+      });
+      *replaced = true;
+      return sync();
+    }
+    return true;
+  }
+
+  // The residual norm of an iteration is folded together with rho of the next
+  // one, after the Z sweep that both need the barrier for; when the norm ends
+  // the loop, that sweep's result is not used.
+  __device__ __forceinline__ bool cg() {
+    const KState &k = sh.k;
+    auto plain_sweep1 = [&](double *r) {
+      sweep1<0>(
+          GVec<double>{r}, [](int) { return 0; }, [](int, int, auto &) {});
+    };
+    plain_sweep1(a.w.r[k.iter & 1]);
+    if (!sync()) return false;
+    bool pending = false;  // the last iteration's norm is not folded yet
+    for (int it = 0; it < a.max_iters || pending;) {
+      const int c = (k.iter + (pending ? 1 : 0)) & 1;
+      double *r = a.w.r[c], *rn = a.w.r[c ^ 1], *p = a.w.p[c], *pn = a.w.p[c ^ 1];
+      const double *norm = gs();
+      if (pending) next_buf();
+      sweep2<1>(
+          a.w.z, [&](int i) { return r[i]; },
+          [&](int, double z, double ri, double (&v)[1]) { v[0] = ri * z; });
+      const double *rho = gs();
+      next_buf();
+      if (!sync()) return false;
+      if (pending) {
+        pending = false;
+        const double *const src[2] = {norm, rho};
+        const bool last = it >= a.max_iters;
+        fold_groups<2>(src, a.ng, sh, [&](const double (&v)[2]) {
+          kstate::finish_iteration(&sh.k, v[0]);
+          sh.rho = v[1];
+          if (!sh.k.done && !periodic_check(sh.k) && !last) kstate::cg_take_rho(&sh.k, v[1]);
+        });
+        if (k.done || periodic_check(k)) {
+          bool replaced;
+          if (!check(r, rn, &replaced)) return false;
+          if (k.done || last) break;
+          if (replaced) {  // t and rho belong to the old r
+            plain_sweep1(r);
+            if (!sync()) return false;
+            continue;
+          }
+          if (threadIdx.x == 0) kstate::cg_take_rho(&sh.k, sh.rho);
+          __syncthreads();
+        } else if (last) {
+          break;
+        }
+      } else {
+        fold_at<1>(rho, [&](const double (&v)[1]) { kstate::cg_take_rho(&sh.k, v[0]); });
+      }
+      if (k.done) break;
+      const GCgP<kB> gp{a.w.z, p, k.beta, k.iter == 0};
+      product<1>(
+          gp, [&](int i) { return gp(i); },
+          [&](int i, double acc, double pi, double (&v)[1]) {
+            pn[i] = pi;
+            a.w.v[i] = acc;
+            v[0] = pi * acc;
+          });
+      if (!sync()) return false;
+      fold<1>([&](const double (&v)[1]) {
+        const double pr[3] = {v[0], 0.0, 0.0};
+        kstate::finish_dots<kCgSigma>(&sh.k, pr, false, nullptr);
+      });
+      if (k.done) break;
+      const double alpha = k.alpha;
+      const GSub<kB> gr{r, a.w.v, alpha};
+      sweep1<1>(
+          gr,
+          [&](int i) { return make_double2(gr(i), a.w.x[i] + alpha * pn[i]); },
+          [&](int i, double2 o, double (&v)[1]) {
+            a.w.x[i] = o.y;
+            rn[i] = o.x;
+            v[0] = o.x * o.x;
+          });
+      if (!sync()) return false;
+      pending = true;
+      it++;
+    }
+    return true;
+  }
+
+  __device__ __forceinline__ bool bicgstab() {
+    const KState &k = sh.k;
+    double *r = a.w.r[0];
+    const auto none = [](int) { return 0; };
+    for (int it = 0; it < a.max_iters && !k.done; it++) {
+      const int c = k.iter & 1;
+      double *p = a.w.p[c], *pn = a.w.p[c ^ 1];
+      const GBiP<kB> gp{r, p, a.w.v, k.beta, k.omega, k.iter == 0};
+      sweep1<0>(
+          gp, [&](int i) { return gp(i); }, [&](int i, double pi, auto &) { pn[i] = pi; });
+      if (!sync()) return false;
+      sweep2<0>(a.w.f, none, [](int, double, int, auto &) {});
+      if (!sync()) return false;
+      product<1>(
+          GVec<double>{a.w.f}, [&](int i) { return a.w.rt[i]; },
+          [&](int i, double acc, double o, double (&v)[1]) {
+            a.w.v[i] = acc;
+            v[0] = o * acc;
+          });
+      if (!sync()) return false;
+      fold<1>([&](const double (&v)[1]) {
+        const double pr[3] = {v[0], 0.0, 0.0};
+        kstate::finish_dots<kBicgSigma>(&sh.k, pr, false, a.w.rt);
+      });
+      if (k.done) break;
+      const double alpha = k.alpha;
+      const GSub<kB> gsv{r, a.w.v, alpha};
+      sweep1<0>(
+          gsv, [&](int i) { return gsv(i); },
+          [&](int i, double si, auto &) { a.w.s[i] = si; });
+      if (!sync()) return false;
+      sweep2<0>(a.w.z, none, [](int, double, int, auto &) {});
+      if (!sync()) return false;
+      product<2>(
+          GVec<double>{a.w.z}, [&](int i) { return a.w.s[i]; },
+          [&](int i, double acc, double o, double (&v)[2]) {
+            a.w.t[i] = acc;
+            v[0] = acc * acc;
+            v[1] = acc * o;
+          });
+      if (!sync()) return false;
+      fold<2>([&](const double (&v)[2]) {
+        const double pr[3] = {v[0], v[1], 0.0};
+        kstate::finish_dots<kBicgOmega>(&sh.k, pr, false, a.w.rt);
+      });
+      if (k.done) break;
+      const double omega = k.omega;
+      groups<2>([&](int, int i, double (&v)[2]) {
+        if (i >= a.n) return;
+        const double xi = (a.w.x[i] + alpha * a.w.f[i]) + omega * a.w.z[i];
+        const double ri = a.w.s[i] - omega * a.w.t[i], rti = a.w.rt[i];
+        a.w.x[i] = xi;
+        r[i] = ri;
+        v[0] = ri * ri;
+        v[1] = rti * ri;
+      });
+      if (!sync()) return false;
+      fold<2>([&](const double (&v)[2]) {
+        kstate::finish_iteration(&sh.k, v[0]);
+        kstate::bicg_next_rho(&sh.k, v[1]);
+      });
+      bool replaced;
+      if (!check(r, p, &replaced)) return false;
+    }
+    return true;
+  }
+};
+
+// One solve (or max_iters iterations of it) by the whole grid.
+template <class V, class T, int K, int METHOD, int MB>
+__global__ void __launch_bounds__(kPBlock, MB) k_persist(PArgs<V, T> a) {
+  __shared__ PShared sh;
+  const int lb = blockIdx.x, nb = gridDim.x;
+  if (threadIdx.x == 0) {
+    sh.k = *a.st;
+    sh.dead = 0;
+    if (lb != 0) sh.k.hist = nullptr;  // block 0 records the residuals
+    if (lb == 0) *a.bar_next = 0u;
+  }
+  __syncthreads();
+  PLoop<V, T, K, METHOD, MB> loop(a, sh, lb, nb);
+  bool ok = a.resume ? true : loop.init();
+  if (ok && !sh.k.done) ok = METHOD == AINV_KRYLOV_CG ? loop.cg() : loop.bicgstab();
+  __syncthreads();
+  if (ok && sh.k.done)
+    loop.template groups<0>([&](int, int row, auto &) {
+      if (row < a.n) a.xout[row] = a.w.x[row];
+    });
+  if (lb == 0 && threadIdx.x == 0) {
+    if (!ok) sh.k.timeout = 1;
+    *a.st = sh.k;
+  }
+}
+
+}  // namespace dev
+}  // namespace ainv
