@@ -62,8 +62,10 @@ struct PMat {
   int lg;  // log2 of the pack
 };
 
-// The vectors of a loop.  r and p alternate: iteration k reads [k & 1] and
-// writes [(k + 1) & 1] (BiCGSTAB keeps r in r[0]).
+// The vectors of a loop.  CG alternates r and p: iteration k reads [k & 1] and
+// writes [(k + 1) & 1].  BiCGSTAB keeps r in r[0] and alternates p, which is in
+// p[0] where a launch starts and ends; p[1] then holds the true residual of a
+// replacement that is still to be done.
 struct PVecs {
   double *x, *b, *r[2], *rt, *p[2], *v, *f, *s, *z, *t;
 };
@@ -502,12 +504,39 @@ struct PLoop {
       kstate::finish_dots<kTrueRes>(&sh.k, v, verify, rt);
     });
     if (k.replace) {
-      groups<0>([&](int, int row, auto &) {
-        if (row < a.n) r[row] = scratch[row];
-      });
       *replaced = true;
-      return sync();
+      return take_r(r, scratch);
     }
+    return true;
+  }
+
+  // r := from, the replacement that the state asks for.
+  __device__ __forceinline__ bool take_r(double *r, const double *from) {
+    groups<0>([&](int, int row, auto &) {
+      if (row < a.n) r[row] = from[row];
+    });
+    const bool ok = sync();
+    if (threadIdx.x == 0) sh.k.replace = 0;
+    return ok;
+  }
+
+  // The solve server's start: x = 0, r = rt = b.
+  __device__ __forceinline__ bool init_zero() {
+    groups<1>([&](int, int i, double (&v)[1]) {
+      if (i >= a.n) return;
+      const double b = a.w.b[i];
+      a.w.x[i] = 0.0;
+      a.w.r[0][i] = b;
+      a.w.rt[i] = b;
+      v[0] = b * b;
+    });
+    if (!sync()) return false;
+    fold<1>([&](const double (&v)[1]) {
+      const double bn = sqrt(v[0]);
+      sh.k.bn2 = (bn == 0.0) ? 1.0 : bn;
+      const double pr[3] = {v[0], v[0], 0.0};
+      kstate::finish_dots<kInit>(&sh.k, pr, false, nullptr);
+    });
     return true;
   }
 
@@ -596,8 +625,10 @@ struct PLoop {
     const KState &k = sh.k;
     double *r = a.w.r[0];
     const auto none = [](int) { return 0; };
-    for (int it = 0; it < a.max_iters && !k.done; it++) {
-      const int c = k.iter & 1;
+    if (k.replace && !take_r(r, a.w.p[1])) return false;
+    int it = 0;
+    for (; it < a.max_iters && !k.done; it++) {
+      const int c = it & 1;
       double *p = a.w.p[c], *pn = a.w.p[c ^ 1];
       const GBiP<kB> gp{r, p, a.w.v, k.beta, k.omega, k.iter == 0};
       sweep1<0>(
@@ -656,6 +687,11 @@ struct PLoop {
       bool replaced;
       if (!check(r, p, &replaced)) return false;
     }
+    // the next launch finds p in p[0]
+    if (!k.done && (it & 1))
+      groups<0>([&](int, int row, auto &) {
+        if (row < a.n) a.w.p[0][row] = a.w.p[1][row];
+      });
     return true;
   }
 };

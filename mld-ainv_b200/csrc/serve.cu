@@ -30,6 +30,9 @@
 // block working for one member, the members' blocks walking the same
 // stages side by side) can be selected per kernel kind.
 //
+// Mixes small enough to be bound by the launches run as one cooperative
+// kernel per step instead (k_srv_persist), with the same iterates.
+//
 // The host side is an engine thread: requests queue on submit, are admitted
 // first-come first-served while a slot is free and their vectors fit in the
 // server's device arena (sized from free HBM at creation), are launched
@@ -51,6 +54,7 @@
 #include <vector>
 
 #include "krylov_epi.cuh"
+#include "persist.cuh"
 
 namespace ainv {
 namespace srv {
@@ -101,11 +105,15 @@ struct Mat {
   const void *val;
   const StageDesc *stages;
   int nstages;
+  int wmax;
+  const int4 *info;
+  const int *pidx;
 };
 
 struct SlotDesc {
   int b0, nb;    // launch blocks [b0, b0 + nb) of the vector kernels
   int fb0, fnb;  // fold blocks [fb0, fb0 + fnb), at most one per range
+  int pb0, pnb;  // persistent loop: blocks [pb0, pb0 + pnb)
   int n, nchunks;
   Mat A, wt, z;
   const void *d;  // D^-1 in the factors' precision
@@ -135,6 +143,7 @@ struct Table {
   short block_slot_f[kMaxGrid];   // folds: the block's slot, -1 idle
   short block_group[kMaxGrid];    // slice-shared operator kernels: the block's group
   short block_group_s[kMaxGrid];  // streamed operator kernels: the block's group
+  short block_slot_p[kMaxGrid];   // persistent loop: the block's slot, -1 idle
 };
 
 struct SlotState {
@@ -144,7 +153,8 @@ struct SlotState {
 };
 
 inline Mat mat_of(const DevSell &m) {
-  return Mat{m.n, m.nslices, m.pack, m.prec, m.sptr, m.iptr, m.idx, m.val, m.stages, m.nstages};
+  return Mat{m.n,    m.nslices, m.pack,    m.prec, m.sptr, m.iptr, m.idx,
+             m.val,  m.stages,  m.nstages, m.wmax, m.info, m.pidx};
 }
 
 // ---------------------------------------------------------------- device --
@@ -869,6 +879,99 @@ __global__ void __launch_bounds__(kStreamThreads, kSrvStreamBlocks)
                            &sts[w.slot].k.timeout, w);
 }
 
+// ---- the persistent loop -----------------------------------------------------------
+// Small mixes are bound by the 14 launches of a batched iteration; then the
+// blocks of one cooperative grid, divided among the slots, run each slot's
+// iterations on their own (persist.cuh), with barriers among the slot's
+// blocks only.  Members of a group do not share the operator's reads here, but
+// operators this small stay in L2.  p is in VP and a pending true residual in
+// VRTRUE at both ends of a launch, as the batched kernels keep them, so the two
+// forms can follow each other.
+constexpr int kPersistBlocks = 2;  // per SM
+// Groups per team up to which a mix runs so (the batched kernels share more
+// reads the more members they have, so they pass it later than a single
+// solve's plain kernels do).  Batch times here / there: one 24^3 request
+// 0.91 / 1.86 ms, 16 of 24^3 and 28^3 2.4 / 6.0, 8 of 31^3 and 48^3 (3.7 groups)
+// 4.5 / 6.8, 16 of 48^3 (11.7) 12.4 / 12.5, 8 of 64^3 (13.8) 17.4 / 16.1.
+constexpr int kPersistPerTeam = 10;
+// Arrival counters and abort words: [parity][slot], on lines of their own.
+constexpr int kBarLine = 32;
+constexpr int kBarWords = 2 * 2 * kMaxSlots * kBarLine;
+__device__ __forceinline__ unsigned *bar_word(unsigned *bars, int what, int parity, int slot) {
+  return bars + ((what * 2 + parity) * kMaxSlots + slot) * kBarLine;
+}
+
+template <class V>
+__device__ __forceinline__ PMat<V> pmat_of(const Mat &m) {
+  return PMat<V>{{m.n, m.nslices, m.info, m.pidx, m.idx, (const V *)m.val}, 31 - __clz(m.pack)};
+}
+
+template <class V, class T, int K>
+__global__ void __launch_bounds__(kPBlock, kPersistBlocks)
+    k_srv_persist(const Table *tab, SlotState *sts, unsigned *bars, int parity, int iters) {
+  __shared__ PShared sh;
+  __shared__ PArgs<V, T> a;
+  // the words of the next launch, for every slot
+  if (blockIdx.x == 0 && threadIdx.x < kMaxSlots) {
+    *bar_word(bars, 0, parity ^ 1, threadIdx.x) = 0u;
+    *bar_word(bars, 1, parity ^ 1, threadIdx.x) = 0u;
+  }
+  const int slot = tab->block_slot_p[blockIdx.x];
+  if (slot < 0) return;
+  SlotState *ss = sts + slot;
+  const int phase = ss->phase;
+  if (phase == kIdle || (phase == kRun && ss->k.done)) return;
+  const SlotDesc &sd = tab->slot[slot];
+  const int lb = blockIdx.x - sd.pb0, nb = sd.pnb;
+  if (threadIdx.x == 0) {
+    sh.k = ss->k;
+    sh.dead = 0;
+    a.wt = pmat_of<V>(sd.wt);
+    a.z = pmat_of<V>(sd.z);
+    a.a = pmat_of<double>(sd.A);
+    a.d = (const V *)sd.d;
+    a.t = (T *)sd.t;
+    a.w = PVecs{sd.vec[VX], sd.vec[VB], {sd.vec[VR], nullptr}, sd.vec[VRT],
+                {sd.vec[VP], sd.vec[VRTRUE]}, sd.vec[VV], sd.vec[VF], sd.vec[VS],
+                sd.vec[VZ], sd.vec[VT]};
+    a.gs = sd.sp;
+    a.n = sd.n;
+    a.ns = sd.ns;
+    a.ng = sd.ng;
+    a.bar = bar_word(bars, 0, parity, slot);
+    a.abort = (int *)bar_word(bars, 1, parity, slot);
+    a.max_iters = iters;
+  }
+  __syncthreads();
+  PLoop<V, T, K, AINV_KRYLOV_BICGSTAB, kPersistBlocks> loop(a, sh, lb, nb);
+  bool ok = phase == kInitPhase ? loop.init_zero() : true;
+  if (ok && !sh.k.done) ok = loop.bicgstab();
+  __syncthreads();
+  if (lb == 0 && threadIdx.x == 0) {
+    if (!ok) sh.k.timeout = 1;
+    ss->k = sh.k;
+    ss->phase = kRun;
+  }
+}
+
+// The kernel for a precision; narrow: factor slices of at most 4 slots.
+void *persist_kernel(int prec, bool narrow) {
+  switch (prec) {
+    case AINV_PREC_FP64:
+      return narrow ? (void *)k_srv_persist<double, double, 4> : (void *)k_srv_persist<double, double, 8>;
+    case AINV_PREC_FP32:
+      return narrow ? (void *)k_srv_persist<float, float, 4> : (void *)k_srv_persist<float, float, 8>;
+    case AINV_PREC_BF16:
+      return narrow ? (void *)k_srv_persist<__nv_bfloat16, float, 4>
+                    : (void *)k_srv_persist<__nv_bfloat16, float, 8>;
+    case AINV_PREC_FP32_ACC64:
+      return narrow ? (void *)k_srv_persist<f32w, double, 4> : (void *)k_srv_persist<f32w, double, 8>;
+    case AINV_PREC_BF16_ACC64:
+      return narrow ? (void *)k_srv_persist<b16w, double, 4> : (void *)k_srv_persist<b16w, double, 8>;
+  }
+  return nullptr;
+}
+
 // ---- launch plan -----------------------------------------------------------------
 enum Family { kFamStd = 1, kFamAcc64 = 2 };
 
@@ -1194,6 +1297,9 @@ struct ainv_server {
   ainv::srv::LaunchPlan plan, graph_plan;   // launches the operators need / in the graph
   int graph_kernels = 0;                    // kernel launches per graph launch
   ainv::srv::SlotState *st_d = nullptr, *st_h = nullptr;
+  unsigned *bars = nullptr;      // persistent loop: arrival counters and abort words
+  int parity = 0;                // which of them the next launch uses
+  void *persist = nullptr;       // kernel for the admitted mix, or null: the graph
   char *arena_d = nullptr;
   ainv::srv::Arena arena;
   std::vector<ainv::srv::Operator> ops;
@@ -1209,7 +1315,7 @@ struct ainv_server {
   std::string error_msg;
   std::chrono::steady_clock::time_point t0;
   // statistics
-  long long submitted = 0, completed = 0, launches = 0;
+  long long submitted = 0, completed = 0, launches = 0, kernels = 0;
   int active = 0, peak_active = 0;
 
   double now() const {
@@ -1382,6 +1488,58 @@ void fill_slot(ainv_server *srv, int k, const Request *r, size_t off) {
   s.phase = kInitPhase;
 }
 
+// Whether the admitted slots run in the persistent loop, and their blocks
+// there: one precision, every matrix within the loop's rows, and no more
+// groups than kPersistPerTeam per team.
+void plan_persist(ainv_server *srv, const std::vector<int> &order) {
+  srv->persist = nullptr;
+  if (order.empty()) return;
+  const int grid = std::min(kMaxGrid, kPersistBlocks * sm_count());
+  if ((int)order.size() > grid) return;
+  const SlotDesc &first = srv->tab_h->slot[order[0]];
+  const bool narrow = first.wt.wmax <= 4 && first.z.wmax <= 4;
+  long long groups = 0;
+  std::vector<long long> w(order.size());
+  std::vector<int> cap(order.size()), b0(order.size()), nb(order.size());
+  for (size_t q = 0; q < order.size(); q++) {
+    const SlotDesc &d = srv->tab_h->slot[order[q]];
+    if (d.smask || d.wt.prec != first.wt.prec || d.n > kPMaxRows ||
+        (d.wt.wmax <= 4 && d.z.wmax <= 4) != narrow)
+      return;
+    groups += d.ng;
+    w[q] = d.ng;
+    cap[q] = (d.ng + kPTeams - 1) / kPTeams;
+  }
+  if (groups > (long long)kPersistPerTeam * kPTeams * grid) return;
+  if (plan_weighted((int)order.size(), w.data(), cap.data(), grid, b0.data(), nb.data()) !=
+      AINV_SUCCESS)
+    return;
+  std::fill(srv->tab_h->block_slot_p, srv->tab_h->block_slot_p + kMaxGrid, (short)-1);
+  for (size_t q = 0; q < order.size(); q++) {
+    SlotDesc &d = srv->tab_h->slot[order[q]];
+    d.pb0 = b0[q];
+    d.pnb = nb[q];
+    for (int b = d.pb0; b < d.pb0 + d.pnb; b++) srv->tab_h->block_slot_p[b] = (short)order[q];
+  }
+  srv->persist = persist_kernel(first.wt.prec, narrow);
+}
+
+// One launch of the persistent loop; false (and the graph from then on, until
+// the mix changes) if the device does not take the grid at once.
+bool launch_persist(ainv_server *srv) {
+  int iters = srv->iters;
+  void *args[] = {&srv->tab_d, &srv->st_d, &srv->bars, &srv->parity, &iters};
+  const int grid = std::min(kMaxGrid, kPersistBlocks * sm_count());
+  if (cudaLaunchCooperativeKernel(srv->persist, dim3(grid), dim3(kPBlock), args, 0, srv->s) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    srv->persist = nullptr;
+    return false;
+  }
+  srv->parity ^= 1;
+  return true;
+}
+
 void engine_loop(ainv_server *srv) {
   cudaSetDevice(srv->device);
   const int S = srv->max_slots;
@@ -1508,21 +1666,27 @@ void engine_loop(ainv_server *srv) {
         gd.nbs = gnb[(size_t)g];
         for (int b = gd.bs0; b < gd.bs0 + gd.nbs; b++) srv->tab_h->block_group_s[b] = (short)g;
       }
+      plan_persist(srv, order);
       ENG_TRY(cudaMemcpyAsync(srv->tab_d, srv->tab_h, sizeof(Table), cudaMemcpyHostToDevice,
                               srv->s));
       dirty = false;
     }
-    LaunchPlan lp;
-    {
-      std::lock_guard<std::mutex> lk(srv->mu);
-      lp = srv->plan;
+    int kernels = 1;
+    if (!srv->persist || !launch_persist(srv)) {
+      LaunchPlan lp;
+      {
+        std::lock_guard<std::mutex> lk(srv->mu);
+        lp = srv->plan;
+      }
+      if (!(lp == srv->graph_plan)) ENG_TRY(capture_graph(srv, lp));  // new operator kinds
+      ENG_TRY(cudaGraphLaunch(srv->exec, srv->s));
+      kernels = srv->graph_kernels;
     }
-    if (!(lp == srv->graph_plan)) ENG_TRY(capture_graph(srv, lp));  // new operator kinds
-    ENG_TRY(cudaGraphLaunch(srv->exec, srv->s));
     ENG_TRY(cudaMemcpyAsync(srv->st_h, srv->st_d, sizeof(SlotState) * (size_t)S,
                             cudaMemcpyDeviceToHost, srv->s));
     ENG_TRY(cudaStreamSynchronize(srv->s));
     srv->launches++;
+    srv->kernels += kernels;
     std::vector<int> done;
     for (int k = 0; k < S; k++) {
       const SlotHost &sl = srv->slots[(size_t)k];
@@ -1636,6 +1800,10 @@ int ainv_server_create(ainv_server **out, int max_slots, size_t hbm_bytes, int i
     return fail(e, "states");
   if ((e = cudaMallocHost(&srv->st_h, sizeof(SlotState) * (size_t)max_slots)) != cudaSuccess)
     return fail(e, "states");
+  if ((e = cudaMalloc(&srv->bars, sizeof(unsigned) * kBarWords)) != cudaSuccess)
+    return fail(e, "counters");
+  if ((e = cudaMemset(srv->bars, 0, sizeof(unsigned) * kBarWords)) != cudaSuccess)
+    return fail(e, "counters");
   if ((e = cudaStreamCreateWithFlags(&srv->s, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(e, "stream");
   std::memset(srv->tab_h, 0, sizeof(Table));
@@ -1643,6 +1811,7 @@ int ainv_server_create(ainv_server **out, int max_slots, size_t hbm_bytes, int i
   std::fill(srv->tab_h->block_slot_f, srv->tab_h->block_slot_f + kMaxGrid, (short)-1);
   std::fill(srv->tab_h->block_group, srv->tab_h->block_group + kMaxGrid, (short)-1);
   std::fill(srv->tab_h->block_group_s, srv->tab_h->block_group_s + kMaxGrid, (short)-1);
+  std::fill(srv->tab_h->block_slot_p, srv->tab_h->block_slot_p + kMaxGrid, (short)-1);
   std::memset(srv->st_h, 0, sizeof(SlotState) * (size_t)max_slots);
   e = cudaMemcpy(srv->tab_d, srv->tab_h, sizeof(Table), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
@@ -1781,7 +1950,7 @@ int ainv_server_stats(ainv_server *srv, ainv_server_info *out) {
   out->submitted = srv->submitted;
   out->completed = srv->completed;
   out->graph_launches = srv->launches;
-  out->kernel_launches = srv->launches * (long long)srv->graph_kernels;
+  out->kernel_launches = srv->kernels;
   out->active = srv->active;
   out->queued = (int)srv->queue.size();
   out->peak_active = srv->peak_active;
@@ -1813,6 +1982,7 @@ int ainv_server_destroy(ainv_server *srv) {
   if (srv->tab_empty_d) cudaFree(srv->tab_empty_d);
   if (srv->tab_h) cudaFreeHost(srv->tab_h);
   if (srv->st_d) cudaFree(srv->st_d);
+  if (srv->bars) cudaFree(srv->bars);
   if (srv->st_h) cudaFreeHost(srv->st_h);
   if (srv->s) cudaStreamDestroy(srv->s);
   delete srv;

@@ -105,3 +105,27 @@ def test_solution_over_right_hand_side():
     both = b.clone()
     A.solve(both, both, f, "CG", 1e-10, 200)
     assert torch.equal(both, x)
+
+
+def test_server_forms_follow_each_other():
+    """Small requests (persistent loop), joined by large ones and by another
+    precision (batched kernels), alone again at the end: every result is the
+    single solve's.  Three iterations per launch, so p changes buffers."""
+    cases = []
+    for idim, prec, kind in [(20, "FP32", "convdiff"), (24, "FP32", "poisson"),
+                             (96, "FP32", "convdiff"), (24, "FP64", "convdiff")]:
+        csr = ainv.pde.gen_pde3d(idim, kind, (6.0, -3.0, 2.0))
+        cases.append((ainv.DeviceOperator(*csr), device_factors(build_factors(*csr), prec), idim ** 3))
+    order = [0, 1, 0, 1, 2, 0, 1, 3, 2, 2, 2, 1, 0, 3, 0, 1]
+    bs = [np.random.default_rng(k).uniform(-1, 1, cases[c][2]) for k, c in enumerate(order)]
+    xs = [np.zeros(cases[c][2]) for c in order]
+    with ainv.SolveServer(max_slots=6, hbm_bytes=1 << 30, iters_per_launch=3) as srv:
+        ops = [srv.add_operator(a, f) for a, f, _ in cases]
+        ids = [srv.submit(ops[c], b, x, 1e-9, 400) for c, b, x in zip(order, bs, xs)]
+        got = [srv.wait(i) for i in ids]
+    for c, b, x, g in zip(order, bs, xs, got):
+        a, f, n = cases[c]
+        ref = torch.zeros(n, dtype=torch.float64, device="cuda")
+        res = a.solve(torch.from_numpy(b).cuda(), ref, f, "BICGSTAB", 1e-9, 400)
+        assert (g.status, g.iter, g.err) == (res.info, res.iter, res.err)
+        np.testing.assert_array_equal(x, ref.cpu().numpy())
