@@ -114,6 +114,7 @@ struct DevSell {
   int4 *info = nullptr;  // nslices
   int *pidx = nullptr;   // offset lists, each padded to a multiple of P
   int wmax = 0;          // widest slice
+  int span = kSlice - 1;  // furthest column a slice reads past its first row (or its last row)
   // streaming stages (see StageDesc); nstages = 0 when not streamable
   int nstages = 0;
   int stage_slices = 0;

@@ -36,9 +36,8 @@ template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
     k_sweep_dscale(InfoView<V> m, const double *__restrict__ x, const V *__restrict__ d,
                    T *__restrict__ t, int s0, int s1, const int *__restrict__ stop) {
-  if (stop && *stop) return;
   for_each_info<P, K>(
-      m, x, s0, s1, [&](int row) { return ldd(d + row); },
+      m, x, s0, s1, [&] { return !stop || !*stop; }, [&](int row) { return ldd(d + row); },
       [&](int row, auto acc, auto dr) { t[row] = (T)(dr * acc); }, [](int) {});
 }
 
@@ -48,11 +47,84 @@ template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
     k_sweep_axpby(InfoView<V> m, const T *__restrict__ t, double alpha, double beta,
                   double *__restrict__ y, int s0, int s1, const int *__restrict__ stop) {
-  if (stop && *stop) return;
   for_each_info<P, K>(
-      m, t, s0, s1, [&](int row) { return beta == 0.0 ? 0.0 : y[row]; },
+      m, t, s0, s1, [&] { return !stop || !*stop; },
+      [&](int row) { return beta == 0.0 ? 0.0 : y[row]; },
       [&](int row, auto acc, double yr) { y[row] = axpby_row(alpha, (double)acc, beta, yr); },
       [](int) {});
+}
+
+// Both sweeps of a small apply in one launch.  Block b owns a tile of slices of
+// the second sweep; it computes every row of t that the tile gathers into
+// shared memory (Z and W are upper triangular: from the tile's first row to
+// `span` rows past its last slice's first), so blocks share nothing and rows of
+// t are computed several times over instead of crossing a grid barrier or a
+// second launch.  The owner also stores its rows of t, as the sweeps do.
+constexpr int kTileBlock = 1024;
+template <class V, class T, int P, int K>
+__global__ void __launch_bounds__(kTileBlock)
+    k_apply_tile(InfoView<V> m1, InfoView<V> m2, const double *__restrict__ x,
+                 const V *__restrict__ d, T *__restrict__ t, double alpha, double beta,
+                 double *__restrict__ y, int tile, int span) {
+  using A = typename Acc<V>::type;
+  constexpr int kStep = kTileBlock / 32;
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  T *tw = reinterpret_cast<T *>(tile_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int a = blockIdx.x * tile, e = min(m1.nslices, a + tile);
+  const int lo = a * kSlice, hi = min(m1.n, (e - 1) * kSlice + span + 1);
+  const int we = (hi + kSlice - 1) / kSlice;  // window: slices [a, we)
+  dep_start();
+  InfoSlab<V, P, K> b;
+  int4 f = make_int4(0, 0, 0, 0);
+  if (a + warp < we) f = __ldg(m1.info + a + warp);
+  info_load(m1, f, 0, b);
+  dep_wait();
+  const auto gx = [&](int c) { return (unsigned)c < (unsigned)m1.n ? __ldg(x + c) : 0.0; };
+  for (int s = a + warp; s < we; s += kStep) {
+    const int row = s * kSlice + lane;
+    const A dr = ldd(d + min(row, m1.n - 1));
+    int4 fn = f;
+    if (s + kStep < we) fn = __ldg(m1.info + s + kStep);
+    A acc = A(0);
+    info_sum<double>(b, f.w ? row : 0, gx, acc);
+    for (int k0 = K; k0 < f.z; k0 += K) {
+      info_load(m1, f, k0, b);
+      info_sum<double>(b, f.w ? row : 0, gx, acc);
+    }
+    f = fn;
+    if (s + kStep < we) info_load(m1, f, 0, b);
+    if (row < hi) {
+      const T tr = (T)(dr * acc);
+      tw[row - lo] = tr;
+      if (s < e) t[row] = tr;
+    }
+  }
+  const int s = a + warp;
+  if (s < e) {
+    f = __ldg(m2.info + s);
+    info_load(m2, f, 0, b);
+  }
+  __syncthreads();
+  const auto gt = [&](int c) {
+    const int i = c - lo;
+    return (unsigned)i < (unsigned)(hi - lo) ? tw[i] : T(0);
+  };
+  for (int q = s; q < e; q += kStep) {
+    const int row = q * kSlice + lane;
+    if (q != s) {
+      f = __ldg(m2.info + q);
+      info_load(m2, f, 0, b);
+    }
+    const double yr = beta == 0.0 ? 0.0 : y[min(row, m2.n - 1)];
+    A acc = A(0);
+    info_sum<T>(b, f.w ? row : 0, gt, acc);
+    for (int k0 = K; k0 < f.z; k0 += K) {
+      info_load(m2, f, k0, b);
+      info_sum<T>(b, f.w ? row : 0, gt, acc);
+    }
+    if (row < m2.n) y[row] = axpby_row(alpha, (double)acc, beta, yr);
+  }
 }
 
 inline int check_launch(const char *what) {
@@ -185,7 +257,7 @@ struct DscaleLaunch {
   template <int P, int K>
   void run() const {
     auto kern = k_sweep_dscale<V, T, P, K>;
-    launch(kern, wave_grid((const void *)kern, (long long)(s1 - s0) * kSlice), kBlock, 0, s,
+    launch_dep(kern, wave_grid((const void *)kern, (long long)(s1 - s0) * kSlice), kBlock, 0, s,
            info_view<V>(m), x, (const V *)d, (T *)t, s0, s1, stop);
   }
 };
@@ -202,8 +274,26 @@ struct AxpbyLaunch {
   template <int P, int K>
   void run() const {
     auto kern = k_sweep_axpby<V, T, P, K>;
-    launch(kern, wave_grid((const void *)kern, (long long)(s1 - s0) * kSlice), kBlock, 0, s,
+    launch_dep(kern, wave_grid((const void *)kern, (long long)(s1 - s0) * kSlice), kBlock, 0, s,
            info_view<V>(m), (const T *)t, alpha, beta, y, s0, s1, stop);
+  }
+};
+
+template <class V, class T>
+struct TileLaunch {
+  const ainv_handle *h;
+  const DevSell &m1, &m2;
+  double alpha, beta;
+  const double *x;
+  double *y;
+  int tile, window;  // slices
+  cudaStream_t s;
+  template <int P>
+  void run() const {
+    if constexpr (P <= 4)
+      launch_dep(k_apply_tile<V, T, P, 4>, (m1.nslices + tile - 1) / tile, kTileBlock,
+                 sizeof(T) * kSlice * (size_t)window, s, info_view<V>(m1), info_view<V>(m2), x,
+                 (const V *)h->d, (T *)h->t, alpha, beta, y, tile, m2.span);
   }
 };
 
@@ -291,20 +381,47 @@ int launch_spmv(const DevSell &a, double alpha, const double *x, double beta, do
   return sweep_axpby(a, x, alpha, beta, y, 0, a.nslices, s, nullptr, "spmv");
 }
 
+// Slices of t that a block of k_apply_tile computes at most: four rounds of
+// its 32 warps.  GPU time here / as two launches, FP64: 24^3 (22 slices) 2.3 /
+// 3.9 us, 40^3 (64) 3.3 / 4.9, 46^3 (88) 4.1 / 5.1, 52^3 (115) 5.0 / 5.7; and a
+// launch less costs the host 1.8 us less per call.  Rows of more than 4 entries
+// are not worth computing several times: INVK(1,1) at 24^3 8.5 / 6.5, at 40^3
+// 19.4 / 9.7.
+constexpr int kTileWindow = 128;
+
+// An apply whose tiles (one per SM) gather few enough rows of t goes out as
+// one launch.  x and y must not overlap: a block reads rows of x that another
+// one owns.
+static bool apply_tile(const ainv_handle *h, const DevSell &m1, const DevSell &m2, double alpha,
+                       const double *x, double beta, double *y, cudaStream_t s) {
+  const int tile = (m1.nslices + sm_count() - 1) / sm_count();
+  const long long window = (long long)tile + m2.span / kSlice + 1;
+  if (window > kTileWindow || m1.pack != m2.pack || m1.wmax > 4 || m2.wmax > 4) return false;
+  const uintptr_t xa = (uintptr_t)x, ya = (uintptr_t)y, nb = sizeof(double) * (uintptr_t)h->n;
+  if (xa < ya + nb && ya < xa + nb) return false;
+  by_prec(m1.prec, [&](auto ty) {
+    using Ty = decltype(ty);
+    with_pack<typename Ty::V>(m1.pack, TileLaunch<typename Ty::V, typename Ty::T>{
+                                           h, m1, m2, alpha, beta, x, y, tile, (int)window, s});
+  });
+  return true;
+}
+
 int ainv_apply_async(const ainv_handle *h, char trans, double alpha, const double *x,
                      double beta, double *y, cudaStream_t s, const int *stop) {
+  bool tr = false;
   switch (trans) {
-    case 'N': case 'n':
-      AINV_TRY(launch_sweep_dscale(h->wt, h->d, x, h->t, s, stop));
-      return launch_sweep_axpby(h->z, h->t, alpha, beta, y, s, stop);
-    case 'T': case 't': case 'C': case 'c':
-      AINV_TRY(launch_sweep_dscale(h->zt, h->d, x, h->t, s, stop));
-      return launch_sweep_axpby(h->w, h->t, alpha, beta, y, s, stop);
+    case 'N': case 'n': break;
+    case 'T': case 't': case 'C': case 'c': tr = true; break;
     default:
       // psb_err_iarg_invalid_i_ (src/impl/mld_d_base_ainv_solver_apply_vect.f90:64-71)
       set_error("invalid trans '%c'", trans);
       return AINV_ERR_ARG;
   }
+  const DevSell &m1 = tr ? h->zt : h->wt, &m2 = tr ? h->w : h->z;
+  if (!stop && apply_tile(h, m1, m2, alpha, x, beta, y, s)) return check_launch("apply");
+  AINV_TRY(launch_sweep_dscale(m1, h->d, x, h->t, s, stop));
+  return launch_sweep_axpby(m2, h->t, alpha, beta, y, s, stop);
 }
 
 }  // namespace ainv

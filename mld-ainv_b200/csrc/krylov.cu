@@ -175,11 +175,10 @@ __global__ void __launch_bounds__(kBlock, info_blocks<double, K>())
     k_spmv_dots(InfoView<double> m, const double *__restrict__ x, double *__restrict__ y,
                 const double *__restrict__ w1, double *__restrict__ w2,
                 const double *__restrict__ w3, const KState *st, SliceOut o) {
-  if (dots_skip<MODE>(st)) return;
   SliceSums<dots_of(MODE)> ss{o.sp, o.ld, {}};
   const double *a = dots_operand<MODE>(x, w1);
   for_each_info<P, K>(
-      m, x, 0, m.nslices, [&](int i) { return a[i]; },
+      m, x, 0, m.nslices, [&] { return !dots_skip<MODE>(st); }, [&](int i) { return a[i]; },
       [&](int i, double acc, double ai) { dots_row<MODE>(i, acc, ai, y, w2, w3, ss); },
       [&](int s) { ss.end(s); });
 }
@@ -197,10 +196,9 @@ template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
     k_cg_sweep2(InfoView<V> m, const T *__restrict__ t, const double *__restrict__ r,
                 double *__restrict__ z, const KState *st, SliceOut o) {
-  if (st->done) return;
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
   for_each_info<P, K>(
-      m, t, 0, m.nslices, [&](int i) { return r[i]; },
+      m, t, 0, m.nslices, [&] { return !st->done; }, [&](int i) { return r[i]; },
       [&](int i, auto acc, double ri) {
         const double zi = (double)acc;
         z[i] = zi;

@@ -261,6 +261,7 @@ int upload_sell_t(const HostCsr &a, int prec, DevSell &out) {
     }
     info[(size_t)s] = make_int4(sptr[s], at, wp, om[s] ? 1 : 0);
     m.wmax = std::max(m.wmax, wp);
+    m.span = std::max(m.span, maxcol[(size_t)s] - s * kSlice);
   }
   m.n = n;
   m.nslices = ns;

@@ -433,6 +433,17 @@ inline InfoView<V> info_view(const DevSell &m) {
   return InfoView<V>{m.n, m.nslices, m.info, m.pidx, m.idx, (const V *)m.val};
 }
 
+// Programmatic dependent launch.  A kernel launched with it (launch_dep) may
+// start while the one before it in the stream still runs: until dep_wait it
+// touches nothing but matrix words, which no kernel writes (D^-1 is not among
+// them: update_a writes it).  Every block waits, so a grid ends after the one
+// before it whatever its blocks do; dep_start lets the next grid's blocks in
+// as this one's leave.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Row `row` of a slice (word group f) dotted with x, K slots at a time.  The
 // gathers of offset-mode slots do not wait for the values: an in-range
 // element is read for zero slots too and replaced by zero, so the products
@@ -513,6 +524,54 @@ __device__ __forceinline__ typename Acc<V>::type info_dot(const InfoView<V> &m, 
   return acc;
 }
 
+// The same in two parts, for a slice whose words are loaded before the vector
+// may be read: K slots of the lane's row (columns relative to the row in
+// offset mode; out of range: not read) ...
+template <class V, int P, int K>
+struct InfoSlab {
+  typename Acc<V>::type v[K / P][P];
+  int c[K / P][P];
+};
+template <class V, int P, int K>
+__device__ __forceinline__ void info_load(const InfoView<V> &m, const int4 &f, int k0,
+                                          InfoSlab<V, P, K> &b) {
+  using A = typename Acc<V>::type;
+  const int lane = threadIdx.x & 31;
+  const int *cp = f.w ? m.pidx + f.y + k0 : m.idx + f.y + k0 * kSlice + lane * P;
+  const int cs = f.w ? P : kSlice * P;
+  const V *vp = m.val + f.x + k0 * kSlice + lane * P;
+#pragma unroll
+  for (int j = 0; j < K / P; j++) {
+    if (k0 + j * P < f.z) {
+      load_ints<P, false>(cp + j * cs, b.c[j]);
+      Pack<V, P>::template load<false>(vp + j * kSlice * P, b.v[j]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < P; e++) {
+        b.c[j][e] = INT_MIN;
+        b.v[j][e] = A(0);
+      }
+    }
+  }
+}
+// ... and acc += their products with the elements g(column) (base: the row in
+// offset mode, else 0).
+template <class X, class V, int P, int K, class G>
+__device__ __forceinline__ void info_sum(const InfoSlab<V, P, K> &b, int base, const G &g,
+                                         typename Acc<V>::type &acc) {
+  using A = typename Acc<V>::type;
+  X xv[K / P][P];
+#pragma unroll
+  for (int j = 0; j < K / P; j++)
+#pragma unroll
+    for (int e = 0; e < P; e++) xv[j][e] = g(b.c[j][e] + base);
+#pragma unroll
+  for (int j = 0; j < K / P; j++)
+#pragma unroll
+    for (int e = 0; e < P; e++)
+      acc = madd(b.v[j][e], b.v[j][e] != A(0) ? (A)xv[j][e] : A(0), acc);
+}
+
 // Slots per step (K of info_dot): 4 where every slice has at most 4 (the AINV
 // and INVT factors of the 7-point operators), else 8 (A has 7, INVK(1,1) 23).
 template <int P>
@@ -522,9 +581,11 @@ constexpr int narrow_k() { return P > 4 ? P : 4; }
 // Narrow steps run best at 6 blocks (40 registers): the 200^3 FP64 apply takes
 // 138, 134, 134 and 173 us at 4, 5, 6 and 8 blocks.  Wide steps need the 64
 // registers of 4 blocks, or spill (100^3 INVK FP64: 71, 76, 86, 84 us), except
-// with 2-byte values (100^3 INVK BF16: 43, 41, 39, 43 us).
+// with BF16 summed in FP32 (100^3 INVK: 43, 41, 39, 43 us).
 template <class V, int K>
-constexpr int info_blocks() { return K <= 4 || sizeof(V) == 2 ? 6 : 4; }
+constexpr int info_blocks() {
+  return K <= 4 || std::is_same<V, __nv_bfloat16>::value ? 6 : 4;
+}
 
 // Call f.template run<P, K>() for a matrix.
 template <class F>
@@ -545,16 +606,21 @@ inline bool with_info(const DevSell &m, const F &f) {
 // Visit the slices [s0, s1), warps striding over the grid, the next slice's
 // word group loaded while this one is summed: pre(row) starts the epilogue's
 // own loads before the sums, post(row, acc, pre's value) runs for rows < n,
-// and end(s) with the whole warp.
-template <int P, int K, class V, class X, class Pre, class Post, class End>
+// and end(s) with the whole warp.  The first slice's words are loaded before
+// dep_wait; go() decides after it whether there is anything to do.
+template <int P, int K, class V, class X, class Go, class Pre, class Post, class End>
 __device__ __forceinline__ void for_each_info(const InfoView<V> &m, const X *__restrict__ x,
-                                              int s0, int s1, Pre &&pre, Post &&post,
+                                              int s0, int s1, Go &&go, Pre &&pre, Post &&post,
                                               End &&end) {
+  using A = typename Acc<V>::type;
   const int lane = threadIdx.x & 31;
   const int step = slice_stride();
   int s = s0 + first_slice();
-  if (s >= s1) return;
-  int4 f = __ldg(m.info + s);
+  dep_start();
+  int4 f = make_int4(0, 0, 0, 0);
+  if (s < s1) f = __ldg(m.info + s);
+  dep_wait();
+  if (s >= s1 || !go()) return;
   for (;;) {
     const int sn = s + step;
     int4 fn = f;
@@ -613,11 +679,24 @@ struct SliceSums {
   }
 };
 
-// k<<<g, b, smem, s>>>(args...) through cudaLaunchKernelEx.  (Launching the
-// apply and Krylov kernels with programmatic dependent launch was measured
-// and dropped: the Krylov iteration did not change, and the early-scheduled
-// blocks of a sweep's successor took shared memory from the persistent
-// streaming sweep, so FP32 and INVK applies lost 20%.)
+// k<<<g, b, smem, s>>>(args...) with programmatic dependent launch, for
+// kernels that call dep_wait.
+template <class... P, class... A>
+inline void launch_dep(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t s, A &&...a) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = g;
+  cfg.blockDim = b;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
+}
+
+// k<<<g, b, smem, s>>>(args...).
 template <class... P, class... A>
 inline void launch(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t s, A &&...a) {
   cudaLaunchConfig_t cfg = {};

@@ -8,7 +8,7 @@ import torch
 
 import ainv
 import oracle as O
-from util import relerr
+from util import build_factors, device_factors, oracle_factors, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +94,61 @@ def test_zero_slots_do_not_read(scattered):
     f.apply(torch.from_numpy(x).cuda(), yd)
     of = O.Factors(O.CSR(n, *wt), O.CSR(n, *z), np.ones(n))
     assert np.array_equal(yd.cpu().numpy(), O.ainv_apply(of, x), equal_nan=True)
+
+
+@pytest.mark.parametrize("idim", [24, 40, 53, 54])
+def test_one_launch_apply(idim):
+    """Grids on both sides of the largest apply that goes out as one launch:
+    the intermediate is left as the sweeps leave it, x and y may be the same
+    vector, and a captured apply can be replayed on new contents."""
+    rng = np.random.default_rng(2)
+    csr = ainv.pde.gen_pde3d(idim, "convdiff", (3.0, 2.0, -1.0))
+    f = build_factors(*csr)
+    n = len(f["d"])
+    df, of = device_factors(f), oracle_factors(f)
+    x1, x2 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    for trans in "NT":
+        x, y = torch.from_numpy(x1).cuda(), torch.zeros(n, dtype=torch.float64, device="cuda")
+        df.apply(x, y, 1.0, 0.0, trans)
+        first = y.clone()
+        assert relerr(first.cpu().numpy(), O.ainv_apply(of, x1, 1.0, 0.0, x1, trans)) <= (
+            0.0 if trans == "N" else 1e-13)
+        df.apply_stage(2, y=y, alpha=2.0, trans=trans)
+        assert torch.equal(y, 2.0 * first)
+        both = x.clone()
+        df.apply(both, both, 1.0, 0.0, trans)
+        assert torch.equal(both, first)
+        part = torch.cat([x, x])
+        df.apply(part[:n], part[n // 2:n // 2 + n], 1.0, 0.0, trans)
+        assert torch.equal(part[n // 2:n // 2 + n], first)
+    x, y = torch.from_numpy(x1).cuda(), torch.zeros(n, dtype=torch.float64, device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        df.apply(x, y, stream=torch.cuda.current_stream())
+        df.apply(y, x, stream=torch.cuda.current_stream())
+    for v in (x1, x2):
+        x.copy_(torch.from_numpy(v))
+        g.replay()
+        torch.cuda.synchronize()
+        once = O.ainv_apply(of, v)
+        assert np.array_equal(y.cpu().numpy(), once)
+        assert np.array_equal(x.cpu().numpy(), O.ainv_apply(of, once))
+
+
+def test_applies_after_update_a():
+    """An apply right behind update_a reads the new diagonal."""
+    csr = ainv.pde.gen_pde3d(24, "poisson")
+    f = build_factors(*csr)
+    n = len(f["d"])
+    x = torch.rand(n, dtype=torch.float64, device="cuda")
+    a, b = device_factors(f), device_factors(f)
+    ya, yb = torch.zeros_like(x), torch.zeros_like(x)
+    a.update_a(x)
+    torch.cuda.synchronize()
+    a.apply(x, ya)
+    b.apply(x, yb)
+    b.update_a(x)
+    b.apply(x, yb)
+    assert torch.equal(ya, yb)
