@@ -41,12 +41,16 @@
 
 namespace ainv {
 
+constexpr int kRecheck = 50;  // true-residual period for FP32/BF16 factors
+
 namespace {
 
 using namespace dev;
 using namespace kstate;
 
-constexpr int kChunk = 8;  // iterations per captured graph launch
+// Iterations per captured graph launch: a divisor of the true-residual period.
+constexpr int kChunk = 10;
+static_assert(kRecheck % kChunk == 0, "periodic checks fall on chunk ends");
 constexpr int kHistCap = 8192;  // iterations whose residual is recorded
 // Arrival counters of the persistent loop, on cache lines of their own.
 constexpr int kBarLine = 32, kBarWords = 3 * kBarLine;
@@ -70,6 +74,8 @@ template <int NV, class Fin>
 __global__ void __launch_bounds__(kFoldThreads)
     k_fold(const double *__restrict__ sp, int ld, int ns, int ng, double *__restrict__ rs,
            int ldr, KState *st, Fin fin) {
+  dep_start();
+  dep_wait();
   if (fin.skip(st)) return;
   __shared__ bool is_last;
   const int nr = gridDim.x;
@@ -155,6 +161,8 @@ __device__ __forceinline__ int nslices_of(int n) { return (n + kSlice - 1) / kSl
 // ||b||_2 (istop=2 denominator).
 __global__ void __launch_bounds__(kBlock)
     k_bnorm(int n, const double *__restrict__ b, SliceOut o) {
+  dep_start();
+  dep_wait();
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
   const int ns = nslices_of(n), lane = threadIdx.x & 31;
   for (int s = first_slice(); s < ns; s += slice_stride()) {
@@ -187,6 +195,8 @@ __global__ void __launch_bounds__(kBlock, info_blocks<double, K>())
 __global__ void __launch_bounds__(kBlock)
     k_replace_r(int n, const double *__restrict__ rtrue, double *__restrict__ r,
                 const KState *st) {
+  dep_start();
+  dep_wait();
   if (!st->replace) return;
   for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) r[i] = rtrue[i];
 }
@@ -211,6 +221,8 @@ __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
 __global__ void __launch_bounds__(kBlock)
     k_cg_ident(int n, const double *__restrict__ r, double *__restrict__ z, const KState *st,
                SliceOut o) {
+  dep_start();
+  dep_wait();
   if (st->done) return;
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
   const int ns = nslices_of(n), lane = threadIdx.x & 31;
@@ -227,6 +239,8 @@ __global__ void __launch_bounds__(kBlock)
 // CG: p = z (first iteration) or p = z + beta p.
 __global__ void __launch_bounds__(kBlock)
     k_cg_p(int n, const double *__restrict__ z, double *__restrict__ p, const KState *st) {
+  dep_start();
+  dep_wait();
   if (st->done) return;
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
@@ -237,6 +251,8 @@ __global__ void __launch_bounds__(kBlock)
 __global__ void __launch_bounds__(kBlock)
     k_cg_xr(int n, const double *__restrict__ p, const double *__restrict__ q,
             double *__restrict__ x, double *__restrict__ r, const KState *st, SliceOut o) {
+  dep_start();
+  dep_wait();
   if (st->done) return;
   const double alpha = st->alpha;
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
@@ -257,6 +273,8 @@ __global__ void __launch_bounds__(kBlock)
 __global__ void __launch_bounds__(kBlock)
     k_bicg_p(int n, const double *__restrict__ r, const double *__restrict__ v,
              double *__restrict__ p, const KState *st) {
+  dep_start();
+  dep_wait();
   if (st->done) return;
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
@@ -267,6 +285,8 @@ __global__ void __launch_bounds__(kBlock)
 __global__ void __launch_bounds__(kBlock)
     k_bicg_s(int n, const double *__restrict__ r, const double *__restrict__ v,
              double *__restrict__ s, const KState *st) {
+  dep_start();
+  dep_wait();
   if (st->done) return;
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= n) return;
@@ -279,6 +299,8 @@ __global__ void __launch_bounds__(kBlock)
               const double *__restrict__ s, const double *__restrict__ t,
               const double *__restrict__ rt, double *__restrict__ x,
               double *__restrict__ r, const KState *st, SliceOut o) {
+  dep_start();
+  dep_wait();
   if (st->done) return;
   const double alpha = st->alpha, omega = st->omega;
   SliceSums<2> ss{o.sp, o.ld, {0.0, 0.0}};
@@ -309,7 +331,7 @@ struct CgSweep2Launch {
   template <int P, int K>
   void run() const {
     auto kern = k_cg_sweep2<V, T, P, K>;
-    launch(kern, wave_grid((const void *)kern, m.n), kBlock, 0, s, info_view<V>(m), (const T *)t,
+    launch_dep(kern, wave_grid((const void *)kern, m.n), kBlock, 0, s, info_view<V>(m), (const T *)t,
            r, z, st, o);
   }
 };
@@ -334,7 +356,7 @@ struct SpmvDotsLaunch {
   template <int P, int K>
   void run() const {
     auto kern = k_spmv_dots<MODE, P, K>;
-    launch(kern, wave_grid((const void *)kern, A.n), kBlock, 0, s, info_view<double>(A), x, y, w1,
+    launch_dep(kern, wave_grid((const void *)kern, A.n), kBlock, 0, s, info_view<double>(A), x, y, w1,
            w2, w3, st, pp);
   }
 };
@@ -376,14 +398,15 @@ struct KrylovWs {
   cudaEvent_t ev = nullptr;
   cudaGraphExec_t exec = nullptr;
   unsigned long long key_serial = 0;
-  int key_method = -1, key_replace = -1;
+  int key_method = -1;
+  bool key_each = false;
   KState last{};  // final state of the last solve (statistics)
   double *v(int i) const { return vec + (size_t)i * stride; }
   SliceOut out() const { return SliceOut{sp, ld, ns}; }
   // Fold the slice sums of the reduction just enqueued (NV dots).
   template <int NV, class Fin>
   void fold(const Fin &fin) const {
-    launch(k_fold<NV, Fin>, nr, kFoldThreads, 0, s, sp, ld, ns, ng, rs, ldr, st, fin);
+    launch_dep(k_fold<NV, Fin>, nr, kFoldThreads, 0, s, sp, ld, ns, ng, rs, ldr, st, fin);
   }
 };
 
@@ -467,8 +490,11 @@ void precond_sweep2_cg(const ainv_handle *h, const double *r, double *z, KState 
 
 // One iteration, enqueued on ws->s.  Kernels ending in a reduction run on
 // the reduction grid G (one resident wave, grid-stride loops); the plain
-// vector updates use one thread per row.
-int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int method) {
+// vector updates use one thread per row.  check: with the true-residual check
+// (three launches that return at once unless convergence is claimed or the
+// period has passed).
+int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int method,
+                      bool check) {
   const int n = w->n, G = w->G;
   const int Gv = (n + kBlock - 1) / kBlock;
   const DevSell &A = a->a;
@@ -482,24 +508,26 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
       AINV_TRY(launch_sweep_dscale(h->wt, h->d, r, h->t, s, stop));
       precond_sweep2_cg(h, r, z, st, pp, s);
     } else {
-      launch(k_cg_ident, std::min(G, wave_grid((const void *)k_cg_ident, n)), kBlock, 0, s, n, r, z,
+      launch_dep(k_cg_ident, std::min(G, wave_grid((const void *)k_cg_ident, n)), kBlock, 0, s, n, r, z,
              st, pp);
     }
     w->fold<1>(FinCgRho{});
-    launch(k_cg_p, Gv, kBlock, 0, s, n, z, p, st);
+    launch_dep(k_cg_p, Gv, kBlock, 0, s, n, z, p, st);
     spmv_dots<kCgSigma>(A, s, p, q, nullptr, nullptr, nullptr, st, pp);
     w->fold<1>(FinDots<kCgSigma>{nullptr});
-    launch(k_cg_xr, std::min(G, wave_grid((const void *)k_cg_xr, n)), kBlock, 0, s, n, p, q, x, r,
+    launch_dep(k_cg_xr, std::min(G, wave_grid((const void *)k_cg_xr, n)), kBlock, 0, s, n, p, q, x, r,
            st, pp);
     w->fold<1>(FinCgXr{});
-    spmv_dots<kTrueRes>(A, s, x, w->v(RTRUE), w->v(BW), nullptr, r, st, pp);
-    w->fold<3>(FinDots<kTrueRes>{nullptr});
-    launch(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n, w->v(RTRUE), r,
-           st);
+    if (check) {
+      spmv_dots<kTrueRes>(A, s, x, w->v(RTRUE), w->v(BW), nullptr, r, st, pp);
+      w->fold<3>(FinDots<kTrueRes>{nullptr});
+      launch_dep(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n,
+                 w->v(RTRUE), r, st);
+    }
   } else {
     double *r = w->v(R), *rt = w->v(RT), *p = w->v(P), *v = w->v(V_), *f = w->v(F),
            *sv = w->v(S), *z = w->v(Z), *t = w->v(T_), *x = w->v(XW);
-    launch(k_bicg_p, Gv, kBlock, 0, s, n, r, v, p, st);
+    launch_dep(k_bicg_p, Gv, kBlock, 0, s, n, r, v, p, st);
     if (h) {
       AINV_TRY(ainv_apply_async(h, 'N', 1.0, p, 0.0, f, s, stop));
     } else {
@@ -507,7 +535,7 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
     }
     spmv_dots<kBicgSigma>(A, s, f, v, rt, nullptr, nullptr, st, pp);
     w->fold<1>(FinDots<kBicgSigma>{rt});
-    launch(k_bicg_s, Gv, kBlock, 0, s, n, r, v, sv, st);
+    launch_dep(k_bicg_s, Gv, kBlock, 0, s, n, r, v, sv, st);
     if (h) {
       AINV_TRY(ainv_apply_async(h, 'N', 1.0, sv, 0.0, z, s, stop));
     } else {
@@ -515,13 +543,15 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
     }
     spmv_dots<kBicgOmega>(A, s, z, t, sv, nullptr, nullptr, st, pp);
     w->fold<2>(FinDots<kBicgOmega>{rt});
-    launch(k_bicg_xr, std::min(G, wave_grid((const void *)k_bicg_xr, n)), kBlock, 0, s, n, f, z, sv,
+    launch_dep(k_bicg_xr, std::min(G, wave_grid((const void *)k_bicg_xr, n)), kBlock, 0, s, n, f, z, sv,
            t, rt, x, r, st, pp);
     w->fold<2>(FinBicgXr{});
-    spmv_dots<kTrueRes>(A, s, x, w->v(RTRUE), w->v(BW), rt, r, st, pp);
-    w->fold<3>(FinDots<kTrueRes>{rt});
-    launch(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n, w->v(RTRUE), r,
-           st);
+    if (check) {
+      spmv_dots<kTrueRes>(A, s, x, w->v(RTRUE), w->v(BW), rt, r, st, pp);
+      w->fold<3>(FinDots<kTrueRes>{rt});
+      launch_dep(k_replace_r, wave_grid((const void *)k_replace_r, n), kBlock, 0, s, n,
+                 w->v(RTRUE), r, st);
+    }
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -531,19 +561,26 @@ int enqueue_iteration(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int 
   return AINV_SUCCESS;
 }
 
-int ensure_graph(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int method,
-                 int replace) {
+// Once the loop is done, nothing of it runs until the check, so a convergence
+// claim can wait for the chunk's end; and as long as no check has failed,
+// chunks start at multiples of kChunk, so the periodic checks fall on their
+// ends.  After a failed claim every iteration is followed by the check.
+int enqueue_chunk(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int method, bool each) {
+  for (int k = 0; k < kChunk; k++)
+    AINV_TRY(enqueue_iteration(w, h, a, method, each || k == kChunk - 1));
+  return AINV_SUCCESS;
+}
+
+int ensure_graph(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int method, bool each) {
   const unsigned long long key = h ? h->serial : 0ull;
-  if (w->exec && w->key_serial == key && w->key_method == method &&
-      w->key_replace == replace)
+  if (w->exec && w->key_serial == key && w->key_method == method && w->key_each == each)
     return AINV_SUCCESS;
   if (w->exec) {
     cudaGraphExecDestroy(w->exec);
     w->exec = nullptr;
   }
   AINV_CUDA_TRY(cudaStreamBeginCapture(w->s, cudaStreamCaptureModeThreadLocal));
-  int rc = AINV_SUCCESS;
-  for (int k = 0; k < kChunk && rc == AINV_SUCCESS; k++) rc = enqueue_iteration(w, h, a, method);
+  const int rc = enqueue_chunk(w, h, a, method, each);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(w->s, &g);
   if (rc != AINV_SUCCESS) {
@@ -563,7 +600,7 @@ int ensure_graph(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, int metho
   }
   w->key_serial = key;
   w->key_method = method;
-  w->key_replace = replace;
+  w->key_each = each;
   return AINV_SUCCESS;
 }
 
@@ -735,7 +772,7 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   AINV_CUDA_TRY(cudaMemcpyAsync(w->v(XW), x, bytes, cudaMemcpyDeviceToDevice, w->s));
   AINV_CUDA_TRY(cudaMemcpyAsync(w->v(BW), b, bytes, cudaMemcpyDeviceToDevice, w->s));
   const DevSell &A = a->a;
-  launch(k_bnorm, std::min(w->G, wave_grid((const void *)k_bnorm, n)), kBlock, 0, w->s, n, w->v(BW),
+  launch_dep(k_bnorm, std::min(w->G, wave_grid((const void *)k_bnorm, n)), kBlock, 0, w->s, n, w->v(BW),
          w->out());
   w->fold<1>(FinBnorm{});
   double *rt0 = method == AINV_KRYLOV_BICGSTAB ? w->v(RT) : nullptr;
@@ -746,16 +783,17 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   // The first chunk always runs as plain launches (kernel attributes are
   // settled outside any capture); later chunks replay one captured graph.
   const bool use_graph = getenv("AINV_NO_GRAPH") == nullptr;
-  const long max_chunks = (long)itmax / kChunk + 2;
+  const long max_chunks = (long)itmax / kChunk + 2 + kMaxVerifyFails;
   for (long c = 0; c < max_chunks; c++) {
     AINV_CUDA_TRY(cudaMemcpyAsync(w->hst, w->st, sizeof(KState), cudaMemcpyDeviceToHost, w->s));
     AINV_CUDA_TRY(cudaStreamSynchronize(w->s));
     if (w->hst->done) break;
+    const bool each = w->hst->fails > 0;
     if (use_graph && c > 0) {
-      AINV_TRY(ensure_graph(w, h, a, method, replace_every));
+      AINV_TRY(ensure_graph(w, h, a, method, each));
       AINV_CUDA_TRY(cudaGraphLaunch(w->exec, w->s));
     } else {
-      for (int k = 0; k < kChunk; k++) AINV_TRY(enqueue_iteration(w, h, a, method));
+      AINV_TRY(enqueue_chunk(w, h, a, method, each));
     }
   }
   AINV_CUDA_TRY(cudaMemcpyAsync(x, w->v(XW), bytes, cudaMemcpyDeviceToDevice, w->s));
@@ -817,7 +855,7 @@ extern "C" int ainv_gpu_solve(ainv_handle *h, const ainv_csr *a, const double *b
   // Every solve confirms convergence on the true residual b - A x.  With
   // FP32/BF16 factors the true residual is also checked every 50 iterations
   // and replaces the recurrence residual if the two have drifted apart.
-  const int replace = (h && h->prec != AINV_PREC_FP64) ? 50 : 0;
+  const int replace = (h && h->prec != AINV_PREC_FP64) ? ainv::kRecheck : 0;
   return ainv::krylov_solve(h, const_cast<ainv_csr *>(a), b_dev, x_dev, method, eps, itmax,
                             replace, iter, err, (cudaStream_t)stream);
 }
