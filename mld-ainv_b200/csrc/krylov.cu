@@ -615,7 +615,7 @@ PMat<V> pmat(const DevSell &m) {
   return PMat<V>{info_view<V>(m), log2i(m.pack)};
 }
 
-template <class V, class T, int K, int METHOD, int MB>
+template <class V, class T, int PK, int K, int METHOD, int MB>
 int persist_launch_mb(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b,
                    double *x, int resume) {
   PArgs<V, T> p;
@@ -645,7 +645,7 @@ int persist_launch_mb(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, cons
   p.st = w->st;
   p.resume = resume;
   p.max_iters = kPersistIters;
-  auto kern = k_persist<V, T, K, METHOD, MB>;
+  auto kern = k_persist<V, T, PK, K, METHOD, MB>;
   static const int per_sm = [&] {
     int v = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, kPBlock, 0) != cudaSuccess) v = 0;
@@ -674,9 +674,12 @@ int persist_launch_mb(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, cons
 template <class V, class T, int K, int METHOD>
 int persist_launch(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b,
                    double *x, int resume) {
-  return w->ng <= kPTeams * sm_count()
-             ? persist_launch_mb<V, T, K, METHOD, 1>(w, h, a, b, x, resume)
-             : persist_launch_mb<V, T, K, METHOD, 2>(w, h, a, b, x, resume);
+  constexpr int PK = fast_pack<V, K>();
+  const bool one = w->ng <= kPTeams * sm_count();  // a group per team, a block per SM
+  if (h->wt.pack == PK && h->z.pack == PK && a->a.pack == 1)
+    return one ? persist_launch_mb<V, T, PK, K, METHOD, 1>(w, h, a, b, x, resume)
+               : persist_launch_mb<V, T, PK, K, METHOD, 2>(w, h, a, b, x, resume);
+  return persist_launch_mb<V, T, 0, K, METHOD, 2>(w, h, a, b, x, resume);
 }
 
 template <int K, int METHOD>

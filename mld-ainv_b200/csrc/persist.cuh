@@ -1,9 +1,9 @@
 // The Krylov loops as one persistent kernel.
 //
-// Below about half a million rows an iteration is bound by its launches, not
+// Below about 600,000 rows an iteration is bound by its launches, not
 // by its bytes: at 40^3 a CG iteration was 11 launches of 2.3-5.5 us (34 us)
 // for 1.7 us of L2 traffic, a BiCGSTAB iteration 20 (52 us).  As phases of
-// one kernel they take 11.2 and 20.8 us: per phase about 0.8 us from the
+// one kernel they take 11.0 and 18.9 us: per phase about 0.8 us from the
 // first gather to the group sums, 1.0 us at the barrier and, where a dot is
 // folded, 1.2 us.  Here the blocks of one cooperative grid run whole
 // iterations, with a grid barrier where one phase reads what another block
@@ -30,7 +30,7 @@
 //
 // Matrix words do not change during the loop.  Up to one group per team the
 // blocks run one per SM with 128 registers, and a warp keeps its slices of
-// the three matrices in them (12.4 -> 11.2 us per CG iteration at 40^3);
+// the three matrices in them (12.4 -> 11.0 us per CG iteration at 40^3);
 // above that, two blocks per SM with 64 registers read them in each phase.
 //
 // Every wait is bounded (kWaitNs); a block that gives up sets the abort word,
@@ -47,11 +47,12 @@ constexpr int kPBufs = 4;   // group-sum buffers used in turn
 constexpr int kPBlock = kPTeams * kFoldThreads;
 constexpr int kPWarps = kPBlock / 32;
 // Groups per team up to which a solve runs here.  Past it a phase is bound by
-// the bytes it moves, and the plain kernels, with 48 warps per SM against 32
-// and wide loads, move them faster: us per iteration here / there at 52^3 CG
-// 16.3 / 33, 64^3 CG 23.9 / 38, 64^3 BiCGSTAB 42.5 / 57 (2 groups), 80^3 CG
-// 42 / 45, 80^3 BiCGSTAB 77 / 73 (4 groups), 100^3 BiCGSTAB 139 / 120.
-constexpr int kPMaxPerTeam = 3;
+// the bytes it moves, and the plain kernels, with 48 warps per SM against 32,
+// move them faster: us per iteration here / there at 52^3 CG 15.1 / 28.6,
+// 64^3 CG 20.0 / 34.0, 64^3 BiCGSTAB 35.4 / 52.3 (2 groups), 80^3 CG 37.4 /
+// 42.9, 80^3 BiCGSTAB 69.8 / 72.3 (4 groups), 90^3 BiCGSTAB 92.9 / 85.9,
+// 100^3 BiCGSTAB 120 / 112.
+constexpr int kPMaxPerTeam = 4;
 // Ranges a block folds in one step (one lane each): 32 ranges of 256 groups.
 constexpr int kPMaxRanges = 32;
 constexpr long long kPMaxRows = (long long)kPMaxRanges * kFoldRange * kGroupSlices * kSlice;
@@ -142,11 +143,16 @@ struct GridBarrier {
 };
 
 // ---- a slice's static words ------------------------------------------------
-// The first K slots of the lane's row: values and columns (-1: not read).
-template <class V, int K>
+// The first K slots of the lane's row.  P: the pack (vector loads), or 0 for
+// any pack (a load per slot, position from the matrix's pack): the phases are
+// bound by the instructions they issue as much as by latency (with P = 0 368
+// per slice and phase at 64^3, 43% of the issue slots; vector loads take the
+// 64^3 BiCGSTAB iteration from 42.5 to 35.4 us).  Copying the values ahead into
+// shared memory (cp.async) cost more instructions than it hid latency: 50 us.
+template <class V, int P, int K>
 struct Slab {
-  typename Acc<V>::type v[K];
-  int c[K];
+  static constexpr int kP = P > 0 ? P : 1;
+  InfoSlab<V, kP, K> b;  // columns relative to the row in offset mode
   int4 f;
 };
 
@@ -154,23 +160,25 @@ __device__ __forceinline__ double ldk(const double *p) { return __ldg(p); }
 template <class V>
 __device__ __forceinline__ typename Acc<V>::type ldk(const V *p) { return ldd(p); }
 
-template <int K, class V>
-__device__ __forceinline__ void slab_slots(const PMat<V> &a, const int4 &f, int row, int k0,
-                                           typename Acc<V>::type (&v)[K], int (&c)[K]) {
-  using A = typename Acc<V>::type;
-  const int lane = threadIdx.x & 31;
-  const int pm = (1 << a.lg) - 1;
+template <class V, int P, int K>
+__device__ __forceinline__ void slab_slots(const PMat<V> &a, const int4 &f, int k0,
+                                           InfoSlab<V, Slab<V, P, K>::kP, K> &b) {
+  if constexpr (P > 0) {
+    info_load(a.m, f, k0, b);
+  } else {
+    const int lane = threadIdx.x & 31;
+    const int pm = (1 << a.lg) - 1;
 #pragma unroll
-  for (int j = 0; j < K; j++) {
-    const int k = k0 + j;
-    if (k < f.z) {
-      const int pos = ((k >> a.lg) << (5 + a.lg)) + (lane << a.lg) + (k & pm);
-      v[j] = ldk(a.m.val + f.x + pos);
-      c[j] = f.w ? row + __ldg(a.m.pidx + f.y + k) : __ldg(a.m.idx + f.y + pos);
-      if ((unsigned)c[j] >= (unsigned)a.m.n) c[j] = -1;
-    } else {
-      v[j] = A(0);
-      c[j] = -1;
+    for (int j = 0; j < K; j++) {
+      const int k = k0 + j;
+      if (k < f.z) {
+        const int pos = ((k >> a.lg) << (5 + a.lg)) + (lane << a.lg) + (k & pm);
+        b.v[j][0] = ldk(a.m.val + f.x + pos);
+        b.c[j][0] = f.w ? __ldg(a.m.pidx + f.y + k) : __ldg(a.m.idx + f.y + pos);
+      } else {
+        b.v[j][0] = 0;
+        b.c[j][0] = INT_MIN;
+      }
     }
   }
 }
@@ -179,52 +187,70 @@ template <class V>
 __device__ __forceinline__ int4 slice_info(const PMat<V> &a, int s) {
   return s < a.m.nslices ? __ldg(a.m.info + s) : make_int4(0, 0, 0, 1);
 }
-template <int K, class V>
-__device__ __forceinline__ void slab_load(const PMat<V> &a, const int4 &f, int row,
-                                          Slab<V, K> &b) {
+template <class V, int P, int K>
+__device__ __forceinline__ void slab_load(const PMat<V> &a, const int4 &f, Slab<V, P, K> &b) {
   b.f = f;
-  slab_slots<K>(a, f, row, 0, b.v, b.c);
+  slab_slots<V, P, K>(a, f, 0, b.b);
 }
 
 // The lane's row dotted with the gathered vector g (g(column) gives an
 // element), G::kBatch gathers in flight; slots in order, zero slots add 0.
-template <class G, int K, class A>
-__device__ __forceinline__ void slab_sum(const A (&v)[K], const int (&c)[K], const G &g, A &acc) {
+template <class V, int P, int K, class G>
+__device__ __forceinline__ void slab_sum(const PMat<V> &a, const InfoSlab<V, P, K> &b, int base,
+                                         const G &g, typename Acc<V>::type &acc) {
+  using A = typename Acc<V>::type;
   constexpr int B = G::kBatch < K ? G::kBatch : K;
 #pragma unroll
   for (int j0 = 0; j0 < K; j0 += B) {
     A xv[B];
 #pragma unroll
-    for (int j = 0; j < B; j++) xv[j] = c[j0 + j] >= 0 ? (A)g(c[j0 + j]) : A(0);
+    for (int j = 0; j < B; j++) {
+      const int c = b.c[(j0 + j) / P][(j0 + j) % P] + base;
+      xv[j] = (unsigned)c < (unsigned)a.m.n ? (A)g(c) : A(0);
+    }
 #pragma unroll
-    for (int j = 0; j < B; j++)
-      acc = madd(v[j0 + j], v[j0 + j] != A(0) ? xv[j] : A(0), acc);
+    for (int j = 0; j < B; j++) {
+      const A v = b.v[(j0 + j) / P][(j0 + j) % P];
+      acc = madd(v, v != A(0) ? xv[j] : A(0), acc);
+    }
   }
 }
 
-template <int K, class V, class G>
-__device__ __forceinline__ typename Acc<V>::type slab_dot(const PMat<V> &a, const Slab<V, K> &b,
-                                                          int row, const G &g) {
-  using A = typename Acc<V>::type;
-  A acc = A(0);
-  slab_sum(b.v, b.c, g, acc);
+template <class V, int P, int K, class G>
+__device__ __forceinline__ typename Acc<V>::type slab_dot(const PMat<V> &a,
+                                                          const Slab<V, P, K> &b, int row,
+                                                          const G &g) {
+  typename Acc<V>::type acc = 0;
+  const int base = b.f.w ? row : 0;
+  slab_sum(a, b.b, base, g, acc);
   for (int k0 = K; k0 < b.f.z; k0 += K) {
-    A v[K];
-    int c[K];
-    slab_slots<K>(a, b.f, row, k0, v, c);
-    slab_sum(v, c, g, acc);
+    InfoSlab<V, Slab<V, P, K>::kP, K> r;
+    slab_slots<V, P, K>(a, b.f, k0, r);
+    slab_sum(a, r, base, g, acc);
   }
   return acc;
 }
 
 // ---- gathered vectors ---------------------------------------------------------
-// Loads are coherent at the barriers (not the read-only path): these vectors
-// are written while the kernel runs.
+// These vectors are written while the kernel runs, so their loads are coherent
+// ones that the compiler must not move across a barrier or reuse after one:
+// volatile (the __ldca and __ldcg intrinsics are functions of the address
+// alone to it).
+__device__ __forceinline__ double ld_now(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_now(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
 template <class X>
 struct GVec {
   static constexpr int kBatch = 8;
   const X *x;
-  __device__ __forceinline__ X operator()(int c) const { return __ldca(x + c); }
+  __device__ __forceinline__ X operator()(int c) const { return ld_now(x + c); }
 };
 // CG: p = z (first iteration) or z + beta p.
 template <int B>
@@ -234,8 +260,8 @@ struct GCgP {
   double beta;
   bool first;
   __device__ __forceinline__ double operator()(int c) const {
-    const double zc = __ldca(z + c);
-    return first ? zc : zc + beta * __ldca(p + c);
+    const double zc = ld_now(z + c);
+    return first ? zc : zc + beta * ld_now(p + c);
   }
 };
 // r - alpha q (CG's r, BiCGSTAB's s).
@@ -245,7 +271,7 @@ struct GSub {
   const double *r, *q;
   double alpha;
   __device__ __forceinline__ double operator()(int c) const {
-    return __ldca(r + c) - alpha * __ldca(q + c);
+    return ld_now(r + c) - alpha * ld_now(q + c);
   }
 };
 // BiCGSTAB: p = r (first iteration) or r + beta (p - omega v).
@@ -256,8 +282,8 @@ struct GBiP {
   double beta, omega;
   bool first;
   __device__ __forceinline__ double operator()(int c) const {
-    const double rc = __ldca(r + c);
-    return first ? rc : rc + beta * (__ldca(p + c) - omega * __ldca(v + c));
+    const double rc = ld_now(r + c);
+    return first ? rc : rc + beta * (ld_now(p + c) - omega * ld_now(v + c));
   }
 };
 
@@ -309,7 +335,7 @@ __device__ __forceinline__ void fold_groups(const double *const (&src)[NV], int 
     for (int q = 0; q < 4; q++) {
       const int g = (u0 + q * kPWarps) * 32 + lane;
 #pragma unroll
-      for (int k = 0; k < NV; k++) v[q][k] = g < ng ? __ldcg(src[k] + g) : 0.0;
+      for (int k = 0; k < NV; k++) v[q][k] = g < ng ? ld_now(src[k] + g) : 0.0;
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -346,17 +372,19 @@ __device__ __forceinline__ bool periodic_check(const KState &k) {
   return !k.done && k.check_every > 0 && k.iter > 0 && k.iter % k.check_every == 0;
 }
 
-template <class V, class T, int K, int METHOD, int MB>
+// P: the pack of W^T and Z with A's pack 1, or 0 for any packs.
+template <class V, class T, int P, int K, int METHOD, int MB>
 struct PLoop {
   static constexpr int KA = 8;  // slots of A per step
+  static constexpr int PA = P > 0 ? 1 : 0;
   static constexpr bool kKeep = MB == 1 && K <= 4;
   static constexpr int kB = MB == 1 ? 8 : 4;  // formed elements in flight
   const PArgs<V, T> &a;
   PShared &sh;
   GridBarrier bar;
   int lb, nb;
-  Slab<V, K> hw, hz;    // the warp's first slice of W^T, Z
-  Slab<double, KA> ha;  // and of A
+  Slab<V, P, K> hw, hz;     // the warp's first slice of W^T, Z
+  Slab<double, PA, KA> ha;  // and of A
   int par = 0;     // group-sum buffer
 
   __device__ __forceinline__ PLoop(const PArgs<V, T> &args, PShared &shared, int lb_, int nb_)
@@ -364,14 +392,13 @@ struct PLoop {
     const int team = threadIdx.x / kFoldThreads;
     const int s0 =
         (lb * kPTeams + team) * kGroupSlices + (int)(threadIdx.x / 32) % kGroupSlices;
-    const int row = s0 * kSlice + (int)(threadIdx.x & 31);
     hw.f = slice_info(a.wt, s0);
     hz.f = slice_info(a.z, s0);
     ha.f = slice_info(a.a, s0);
     if constexpr (kKeep) {
-      slab_load<K>(a.wt, hw.f, row, hw);
-      slab_load<K>(a.z, hz.f, row, hz);
-      slab_load<KA>(a.a, ha.f, row, ha);
+      slab_load(a.wt, hw.f, hw);
+      slab_load(a.z, hz.f, hz);
+      slab_load(a.a, ha.f, ha);
     }
   }
   __device__ __forceinline__ double *gs() const { return a.gs + (size_t)par * 3 * a.ng; }
@@ -401,8 +428,8 @@ struct PLoop {
   // (h) is kept in registers through the loop where they suffice (kKeep:
   // most systems have one group per team there), else its word group is;
   // the next slice's word group is loaded while this slice is summed.
-  template <int NV, int KK, class U, class Body>
-  __device__ __forceinline__ void slabs(const PMat<U> &m, const Slab<U, KK> &h, Body &&body) {
+  template <int NV, class U, int PP, int KK, class Body>
+  __device__ __forceinline__ void slabs(const PMat<U> &m, const Slab<U, PP, KK> &h, Body &&body) {
     int4 f = h.f;
     bool head = true;
     groups<NV>([&](int s, int row, auto &v) {
@@ -410,8 +437,8 @@ struct PLoop {
       if (kKeep && head) {
         body(row, h, v);
       } else {
-        Slab<U, KK> b;
-        slab_load<KK>(m, f, row, b);
+        Slab<U, PP, KK> b;
+        slab_load(m, f, b);
         body(row, b, v);
       }
       head = false;
@@ -424,10 +451,10 @@ struct PLoop {
   // t = D^-1 W^T g.
   template <int NV, class G, class Pre, class Post>
   __device__ __forceinline__ void sweep1(const G &g, Pre &&pre, Post &&post) {
-    slabs<NV, K>(a.wt, hw, [&](int row, const Slab<V, K> &b, auto &v) {
+    slabs<NV>(a.wt, hw, [&](int row, const auto &b, auto &v) {
       const auto o = pre(clamp(row));
       const auto d = ldk(a.d + clamp(row));
-      const auto acc = slab_dot<K>(a.wt, b, row, g);
+      const auto acc = slab_dot(a.wt, b, row, g);
       if (row < a.n) {
         a.t[row] = (T)(d * acc);
         post(row, o, v);
@@ -438,9 +465,9 @@ struct PLoop {
   template <int NV, class Pre, class Post>
   __device__ __forceinline__ void sweep2(double *dst, Pre &&pre, Post &&post) {
     const GVec<T> g{a.t};
-    slabs<NV, K>(a.z, hz, [&](int row, const Slab<V, K> &b, auto &v) {
+    slabs<NV>(a.z, hz, [&](int row, const auto &b, auto &v) {
       const auto o = pre(clamp(row));
-      const auto acc = slab_dot<K>(a.z, b, row, g);
+      const auto acc = slab_dot(a.z, b, row, g);
       if (row < a.n) {
         const double z = (double)acc;
         dst[row] = z;
@@ -451,9 +478,9 @@ struct PLoop {
   // (A g)[row] for post.
   template <int NV, class G, class Pre, class Post>
   __device__ __forceinline__ void product(const G &g, Pre &&pre, Post &&post) {
-    slabs<NV, KA>(a.a, ha, [&](int row, const Slab<double, KA> &b, auto &v) {
+    slabs<NV>(a.a, ha, [&](int row, const auto &b, auto &v) {
       const auto o = pre(clamp(row));
-      const double acc = slab_dot<KA>(a.a, b, row, g);
+      const double acc = slab_dot(a.a, b, row, g);
       if (row < a.n) post(row, acc, o, v);
     });
   }
@@ -696,8 +723,15 @@ struct PLoop {
   }
 };
 
+// The pack that most matrices of a width class get (layout.cpp), the one with
+// kernels of its own.
+template <class V, int K>
+constexpr int fast_pack() {
+  return sizeof(V) == 8 ? 2 : sizeof(V) == 4 || K <= 4 ? 4 : 8;
+}
+
 // One solve (or max_iters iterations of it) by the whole grid.
-template <class V, class T, int K, int METHOD, int MB>
+template <class V, class T, int P, int K, int METHOD, int MB>
 __global__ void __launch_bounds__(kPBlock, MB) k_persist(PArgs<V, T> a) {
   __shared__ PShared sh;
   const int lb = blockIdx.x, nb = gridDim.x;
@@ -708,7 +742,7 @@ __global__ void __launch_bounds__(kPBlock, MB) k_persist(PArgs<V, T> a) {
     if (lb == 0) *a.bar_next = 0u;
   }
   __syncthreads();
-  PLoop<V, T, K, METHOD, MB> loop(a, sh, lb, nb);
+  PLoop<V, T, P, K, METHOD, MB> loop(a, sh, lb, nb);
   bool ok = a.resume ? true : loop.init();
   if (ok && !sh.k.done) ok = METHOD == AINV_KRYLOV_CG ? loop.cg() : loop.bicgstab();
   __syncthreads();

@@ -888,12 +888,12 @@ __global__ void __launch_bounds__(kStreamThreads, kSrvStreamBlocks)
 // VRTRUE at both ends of a launch, as the batched kernels keep them, so the two
 // forms can follow each other.
 constexpr int kPersistBlocks = 2;  // per SM
-// Groups per team up to which a mix runs so (the batched kernels share more
-// reads the more members they have, so they pass it later than a single
-// solve's plain kernels do).  Batch times here / there: one 24^3 request
-// 0.91 / 1.86 ms, 16 of 24^3 and 28^3 2.4 / 6.0, 8 of 31^3 and 48^3 (3.7 groups)
-// 4.5 / 6.8, 16 of 48^3 (11.7) 12.4 / 12.5, 8 of 64^3 (13.8) 17.4 / 16.1.
-constexpr int kPersistPerTeam = 10;
+// Groups per team up to which a mix runs so.  Batch times here / there: one
+// 24^3 request 0.80 / 1.85 ms, 16 of 24^3 and 28^3 2.1 / 6.2, 8 of 31^3 and 48^3
+// (3.7 groups) 3.7 / 6.8, 16 of 48^3 (11.7) 9.5 / 12.4, 8 of 64^3 (13.8) 14.1 /
+// 16.7, 16 of 64^3 (27.7) 26.7 / 27.3; past that the two are level, and the
+// batched kernels share an operator's reads.
+constexpr int kPersistPerTeam = 32;
 // Arrival counters and abort words: [parity][slot], on lines of their own.
 constexpr int kBarLine = 32;
 constexpr int kBarWords = 2 * 2 * kMaxSlots * kBarLine;
@@ -906,7 +906,7 @@ __device__ __forceinline__ PMat<V> pmat_of(const Mat &m) {
   return PMat<V>{{m.n, m.nslices, m.info, m.pidx, m.idx, (const V *)m.val}, 31 - __clz(m.pack)};
 }
 
-template <class V, class T, int K>
+template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kPBlock, kPersistBlocks)
     k_srv_persist(const Table *tab, SlotState *sts, unsigned *bars, int parity, int iters) {
   __shared__ PShared sh;
@@ -943,7 +943,7 @@ __global__ void __launch_bounds__(kPBlock, kPersistBlocks)
     a.max_iters = iters;
   }
   __syncthreads();
-  PLoop<V, T, K, AINV_KRYLOV_BICGSTAB, kPersistBlocks> loop(a, sh, lb, nb);
+  PLoop<V, T, P, K, AINV_KRYLOV_BICGSTAB, kPersistBlocks> loop(a, sh, lb, nb);
   bool ok = phase == kInitPhase ? loop.init_zero() : true;
   if (ok && !sh.k.done) ok = loop.bicgstab();
   __syncthreads();
@@ -954,20 +954,27 @@ __global__ void __launch_bounds__(kPBlock, kPersistBlocks)
   }
 }
 
-// The kernel for a precision; narrow: factor slices of at most 4 slots.
-void *persist_kernel(int prec, bool narrow) {
+// The kernel for a precision; narrow: factor slices of at most 4 slots; fast:
+// the packs that have kernels of their own.
+template <class V, class T, int K>
+void *persist_kernel_k(bool fast) {
+  return fast ? (void *)k_srv_persist<V, T, fast_pack<V, K>(), K> : (void *)k_srv_persist<V, T, 0, K>;
+}
+template <class V, class T>
+void *persist_kernel_v(bool narrow, const SlotDesc *const *d, size_t n) {
+  const int P = narrow ? fast_pack<V, 4>() : fast_pack<V, 8>();
+  bool fast = true;
+  for (size_t q = 0; q < n; q++)
+    fast = fast && d[q]->wt.pack == P && d[q]->z.pack == P && d[q]->A.pack == 1;
+  return narrow ? persist_kernel_k<V, T, 4>(fast) : persist_kernel_k<V, T, 8>(fast);
+}
+void *persist_kernel(int prec, bool narrow, const SlotDesc *const *d, size_t n) {
   switch (prec) {
-    case AINV_PREC_FP64:
-      return narrow ? (void *)k_srv_persist<double, double, 4> : (void *)k_srv_persist<double, double, 8>;
-    case AINV_PREC_FP32:
-      return narrow ? (void *)k_srv_persist<float, float, 4> : (void *)k_srv_persist<float, float, 8>;
-    case AINV_PREC_BF16:
-      return narrow ? (void *)k_srv_persist<__nv_bfloat16, float, 4>
-                    : (void *)k_srv_persist<__nv_bfloat16, float, 8>;
-    case AINV_PREC_FP32_ACC64:
-      return narrow ? (void *)k_srv_persist<f32w, double, 4> : (void *)k_srv_persist<f32w, double, 8>;
-    case AINV_PREC_BF16_ACC64:
-      return narrow ? (void *)k_srv_persist<b16w, double, 4> : (void *)k_srv_persist<b16w, double, 8>;
+    case AINV_PREC_FP64: return persist_kernel_v<double, double>(narrow, d, n);
+    case AINV_PREC_FP32: return persist_kernel_v<float, float>(narrow, d, n);
+    case AINV_PREC_BF16: return persist_kernel_v<__nv_bfloat16, float>(narrow, d, n);
+    case AINV_PREC_FP32_ACC64: return persist_kernel_v<f32w, double>(narrow, d, n);
+    case AINV_PREC_BF16_ACC64: return persist_kernel_v<b16w, double>(narrow, d, n);
   }
   return nullptr;
 }
@@ -1501,8 +1508,10 @@ void plan_persist(ainv_server *srv, const std::vector<int> &order) {
   long long groups = 0;
   std::vector<long long> w(order.size());
   std::vector<int> cap(order.size()), b0(order.size()), nb(order.size());
+  std::vector<const SlotDesc *> descs(order.size());
   for (size_t q = 0; q < order.size(); q++) {
     const SlotDesc &d = srv->tab_h->slot[order[q]];
+    descs[q] = &d;
     if (d.smask || d.wt.prec != first.wt.prec || d.n > kPMaxRows ||
         (d.wt.wmax <= 4 && d.z.wmax <= 4) != narrow)
       return;
@@ -1521,7 +1530,7 @@ void plan_persist(ainv_server *srv, const std::vector<int> &order) {
     d.pnb = nb[q];
     for (int b = d.pb0; b < d.pb0 + d.pnb; b++) srv->tab_h->block_slot_p[b] = (short)order[q];
   }
-  srv->persist = persist_kernel(first.wt.prec, narrow);
+  srv->persist = persist_kernel(first.wt.prec, narrow, descs.data(), descs.size());
 }
 
 // One launch of the persistent loop; false (and the graph from then on, until

@@ -129,3 +129,28 @@ def test_server_forms_follow_each_other():
         res = a.solve(torch.from_numpy(b).cuda(), ref, f, "BICGSTAB", 1e-9, 400)
         assert (g.status, g.iter, g.err) == (res.info, res.iter, res.err)
         np.testing.assert_array_equal(x, ref.cpu().numpy())
+
+
+@pytest.mark.parametrize("method,idim", [("CG", 84), ("BICGSTAB", 84), ("BICGSTAB", 85)])
+def test_largest(method, idim):
+    """The largest grid of the persistent loop, and the first of the plain one."""
+    kind = "poisson" if method == "CG" else "convdiff"
+    csr = ainv.pde.gen_pde3d(idim, kind, (4.0, -3.0, 2.0))
+    check(method, csr, build_factors(*csr))
+
+
+@pytest.mark.parametrize("method", ["CG", "BICGSTAB"])
+@pytest.mark.parametrize("offs", [(-1, 0, 1), (-40, -1, 0, 1, 40, 41), (-3, 0, 1, 7)])
+def test_other_packs(method, offs):
+    """Operators and factors whose layout packs differ from those with kernels
+    of their own (slices of 2, 3, 4 and 6 slots)."""
+    rng = np.random.default_rng(4)
+    n = 5000
+    irp, ja, val = [0], [], []
+    for r in range(n):
+        cols = [r + o for o in offs if 0 <= r + o < n]
+        ja += cols
+        val += [8.0 if c == r else -1.0 + 0.1 * rng.random() for c in cols]
+        irp.append(len(ja))
+    csr = np.array(irp, np.int32), np.array(ja, np.int32), np.array(val)
+    check(method, csr, build_factors(*csr))
