@@ -55,123 +55,161 @@ struct MState {
 
 // ---------------------------------------------------------------- device --
 // Lane map of the SpMM kernels: a warp works on 4 rows of a slice at a time,
-// lane = 8 q + g takes row q of the four and columns 4g .. 4g+3, so the 8
-// lanes of a row read its 32 columns as one 256-byte line (32 bytes each).
+// lane = 8 q + g takes row q of the four and 4 of its columns, so the 8 lanes
+// of a row read its 32 columns as one 256-byte line.
 constexpr int kColsPerLane = 4;
 constexpr int kRowsPerStep = kSlice / 8;  // 4
 constexpr int kSlotBatch = 4;
 
-__device__ __forceinline__ void ldg4(const double *p, double (&o)[4]) {
-  const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
-  const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-  o[0] = a.x;
-  o[1] = a.y;
-  o[2] = b.x;
-  o[3] = b.y;
-}
-__device__ __forceinline__ void ldg4(const float *p, float (&o)[4]) {
-  const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-  o[0] = a.x;
-  o[1] = a.y;
-  o[2] = a.z;
-  o[3] = a.w;
-}
-__device__ __forceinline__ void ld4(const double *p, double (&o)[4]) {
-  const double2 a = reinterpret_cast<const double2 *>(p)[0];
-  const double2 b = reinterpret_cast<const double2 *>(p)[1];
-  o[0] = a.x;
-  o[1] = a.y;
-  o[2] = b.x;
-  o[3] = b.y;
-}
-__device__ __forceinline__ void st4(double *p, const double (&v)[4]) {
-  reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
-  reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
-}
-__device__ __forceinline__ void st4(float *p, const float (&v)[4]) {
-  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-// Evict-first stores for the products' multivector outputs (Q, T, Z): they
-// are larger than L2 and read back only by a later kernel, so they should
-// not displace the gathered input's rows that the next slices reuse.
-__device__ __forceinline__ void st4cs(double *p, const double (&v)[4]) {
-  __stcs(reinterpret_cast<double2 *>(p), make_double2(v[0], v[1]));
-  __stcs(reinterpret_cast<double2 *>(p) + 1, make_double2(v[2], v[3]));
-}
-__device__ __forceinline__ void st4cs(float *p, const float (&v)[4]) {
-  __stcs(reinterpret_cast<float4 *>(p), make_float4(v[0], v[1], v[2], v[3]));
-}
-
-// acc[e] = row `row` (slice-local rs) of M times column c0 + e of x.  Slots
-// are taken kSlotBatch at a time: their values and index words load
-// together, then the batch's gathers (skipped where the value is 0) are all
-// in flight before the first fma.  Slot order and fma sequence per (row,
-// column) are those of the single-vector kernels.
-template <class V, class X, class A>
-__device__ __forceinline__ void row_mm(const SellView<V> &m, int pack, int vb, int ib, int w,
-                                       bool om, int row, int rs, const X *__restrict__ x, int c0,
-                                       A (&acc)[kColsPerLane]) {
-#pragma unroll
-  for (int e = 0; e < kColsPerLane; e++) acc[e] = A(0);
-  for (int k0 = 0; k0 < w; k0 += kSlotBatch) {
-    A v[kSlotBatch];
-    int c[kSlotBatch];
-#pragma unroll
-    for (int j = 0; j < kSlotBatch; j++) {
-      const int k = k0 + j;
-      if (k < w) {
-        const int pos = (k / pack) * (kSlice * pack) + rs * pack + (k % pack);
-        v[j] = (A)ldv(m.val + vb + pos);
-        c[j] = om ? row + __ldg(m.idx + ib + k) : __ldcs(m.idx + ib + pos);
-      } else {
-        v[j] = A(0);
-        c[j] = 0;
-      }
-    }
-    A xv[kSlotBatch][kColsPerLane];
-#pragma unroll
-    for (int j = 0; j < kSlotBatch; j++) {
-      if (v[j] != A(0) && (unsigned)c[j] < (unsigned)m.n) {
-        X t[kColsPerLane];
-        ldg4(x + (size_t)c[j] * kCols + c0, t);
-#pragma unroll
-        for (int e = 0; e < kColsPerLane; e++) xv[j][e] = (A)t[e];
-      } else {
-#pragma unroll
-        for (int e = 0; e < kColsPerLane; e++) xv[j][e] = A(0);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kSlotBatch; j++)
-#pragma unroll
-      for (int e = 0; e < kColsPerLane; e++) acc[e] = madd(v[j], xv[j][e], acc[e]);
+// The 4 columns of lane g.  SPLIT: 2g, 2g+1, 16+2g, 17+2g, so that each of the
+// two 16-byte accesses that FP64 rows need covers 128 contiguous bytes of the
+// row; else 4g .. 4g+3, one 16-byte access of an FP32 row.  (With 4g for FP64
+// both accesses touch both lines of the row: l1tex at 74% of its peak in the A
+// product, split 51%.)
+template <bool SPLIT>
+struct Cols {
+  int g;
+  __device__ __forceinline__ int at(int e) const {
+    return SPLIT ? (e & 2) * 8 + 2 * g + (e & 1) : 4 * g + e;
   }
+  // the two halves' offsets in a row
+  __device__ __forceinline__ int lo() const { return SPLIT ? 2 * g : 4 * g; }
+  __device__ __forceinline__ int hi() const { return SPLIT ? 16 + 2 * g : 4 * g + 2; }
+  __device__ __forceinline__ void ldg(const double *row, double (&o)[4]) const {
+    const double2 a = __ldg(reinterpret_cast<const double2 *>(row + lo()));
+    const double2 b = __ldg(reinterpret_cast<const double2 *>(row + hi()));
+    o[0] = a.x;
+    o[1] = a.y;
+    o[2] = b.x;
+    o[3] = b.y;
+  }
+  __device__ __forceinline__ void ldg(const float *row, float (&o)[4]) const {
+    static_assert(!SPLIT, "FP32 rows are gathered unsplit");
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(row + 4 * g));
+    o[0] = a.x;
+    o[1] = a.y;
+    o[2] = a.z;
+    o[3] = a.w;
+  }
+  __device__ __forceinline__ void st(double *row, const double (&v)[4]) const {
+    *reinterpret_cast<double2 *>(row + lo()) = make_double2(v[0], v[1]);
+    *reinterpret_cast<double2 *>(row + hi()) = make_double2(v[2], v[3]);
+  }
+  // Evict-first stores for the products' multivector outputs (Q, T, Z): they
+  // are larger than L2 and read back only by a later kernel, so they should
+  // not displace the gathered input's rows that the next slices reuse.
+  __device__ __forceinline__ void stcs(double *row, const double (&v)[4]) const {
+    __stcs(reinterpret_cast<double2 *>(row + lo()), make_double2(v[0], v[1]));
+    __stcs(reinterpret_cast<double2 *>(row + hi()), make_double2(v[2], v[3]));
+  }
+  __device__ __forceinline__ void stcs(float *row, const float (&v)[4]) const {
+    if constexpr (SPLIT) {
+      __stcs(reinterpret_cast<float2 *>(row + lo()), make_float2(v[0], v[1]));
+      __stcs(reinterpret_cast<float2 *>(row + hi()), make_float2(v[2], v[3]));
+    } else {
+      __stcs(reinterpret_cast<float4 *>(row + 4 * g), make_float4(v[0], v[1], v[2], v[3]));
+    }
+  }
+};
+// The column map of a kernel that gathers rows of X.
+template <class X>
+using ColsOf = Cols<sizeof(X) == 8>;
+
+// Add slots [k0, k0 + NB) of a row to acc: v[j], c[j] its values and columns.
+// The batch's gathers are all in flight before the first product and do not
+// wait for the values: an in-range row is read for zero slots too and replaced
+// by zero.
+template <int NB, class X, class A>
+__device__ __forceinline__ void add_slots(int n, const A (&v)[NB], const int (&c)[NB],
+                                          const X *__restrict__ x, const ColsOf<X> &cm,
+                                          A (&acc)[kColsPerLane]) {
+  X xv[NB][kColsPerLane];
+#pragma unroll
+  for (int j = 0; j < NB; j++) {
+#pragma unroll
+    for (int e = 0; e < kColsPerLane; e++) xv[j][e] = X(0);
+    if ((unsigned)c[j] < (unsigned)n) cm.ldg(x + (size_t)c[j] * kCols, xv[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < NB; j++)
+#pragma unroll
+    for (int e = 0; e < kColsPerLane; e++)
+      acc[e] = madd(v[j], v[j] != A(0) ? (A)xv[j][e] : A(0), acc[e]);
 }
 
-// Visit every row of M (warps striding over slices): epi(row, c0, acc) with
-// the thread's 4 columns; each thread's rows come in ascending order.  (A
-// contiguous run of slices per warp, which spreads the warps' fronts over
-// the matrix, measured slower at 128^3 x 32: 0.604 against 0.497 s per
-// block solve.)
-template <class V, class X, class Epi>
-__device__ __forceinline__ void for_each_slice(const SellView<V> &m, int pack,
-                                               const X *__restrict__ x, Epi &&epi) {
+// Visit every row of M (warps striding over slices): epi(e0, columns, acc) with
+// the row's first element and the thread's 4 columns; each thread's rows come
+// in ascending order.  (A contiguous run of slices per warp, which spreads the
+// warps' fronts over the matrix, measured slower at 128^3 x 32: 0.604 against
+// 0.497 s per block solve.)  A slice's first K slots are loaded once, each
+// lane those of its own row, and passed to the lanes that work on the row by
+// shuffles: the gathers of the 8 steps then wait for no other load.  Loading
+// values and columns in every step made two dependent loads of it (block
+// solves with 32 right-hand sides and FP32 factors then / now: 24^3 4.6 / 4.2
+// ms, 64^3 34.9 / 32.6, 100^3 152 / 145).  What bounds it now is the latency of
+// the gathers (28 warps per SM, DRAM at 1.5 TB/s in the A product at 64^3).
+// Slot order and products per (row, column) are those of the single-vector
+// kernels.
+template <int P, int K, class V, class X, class Epi>
+__device__ __forceinline__ void for_each_slice(const InfoView<V> &m, const X *__restrict__ x,
+                                               Epi &&epi) {
   using A = typename Acc<V>::type;
+  constexpr int NB = kSlotBatch;
   const int lane = threadIdx.x & 31;
-  const int q = lane >> 3, c0 = (lane & 7) * kColsPerLane;
-  for (int s = first_slice(); s < m.nslices; s += slice_stride()) {
-    const int vb = __ldg(m.sptr + s), ve = __ldg(m.sptr + s + 1);
-    const int ib = __ldg(m.iptr + s), ie = __ldg(m.iptr + s + 1);
-    const int w = (ve - vb) / kSlice;
-    const bool om = (ie - ib) == w;
+  const int q = lane >> 3;
+  const ColsOf<X> cm{lane & 7};
+  int s = first_slice();
+  if (s >= m.nslices) return;
+  int4 f = __ldg(m.info + s);
+  for (;;) {
+    const int sn = s + slice_stride();
+    int4 fn = f;
+    if (sn < m.nslices) fn = __ldg(m.info + sn);
+    InfoSlab<V, P, K> b;
+    info_load(m, f, 0, b);
 #pragma unroll 2
     for (int t = 0; t < kSlice / kRowsPerStep; t++) {
       const int rs = t * kRowsPerStep + q;
       const int row = s * kSlice + rs;
       A acc[kColsPerLane];
-      row_mm(m, pack, vb, ib, w, om, row, rs, x, c0, acc);
-      if (row < m.n) epi(row, c0, acc);
+#pragma unroll
+      for (int e = 0; e < kColsPerLane; e++) acc[e] = A(0);
+#pragma unroll
+      for (int k0 = 0; k0 < K; k0 += NB) {
+        if (k0 < f.z) {
+          A v[NB];
+          int c[NB];
+#pragma unroll
+          for (int j = 0; j < NB; j++) {
+            const int k = k0 + j;
+            v[j] = __shfl_sync(0xffffffffu, b.v[k / P][k % P], rs);
+            c[j] = f.w ? row + b.c[k / P][k % P]
+                       : __shfl_sync(0xffffffffu, b.c[k / P][k % P], rs);
+          }
+          add_slots<NB>(m.n, v, c, x, cm, acc);
+        }
+      }
+      for (int k0 = K; k0 < f.z; k0 += NB) {
+        A v[NB];
+        int c[NB];
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+          const int k = k0 + j;
+          v[j] = A(0);
+          c[j] = -1;
+          if (k < f.z) {
+            const int pos = (k / P) * (kSlice * P) + rs * P + k % P;
+            v[j] = (A)ldv(m.val + f.x + pos);
+            c[j] = f.w ? row + __ldg(m.pidx + f.y + k) : __ldcs(m.idx + f.y + pos);
+          }
+        }
+        add_slots<NB>(m.n, v, c, x, cm, acc);
+      }
+      if (row < m.n) epi((size_t)row * kCols, cm, acc);
     }
+    if (sn >= m.nslices) break;
+    s = sn;
+    f = fn;
   }
 }
 
@@ -235,18 +273,19 @@ __device__ __forceinline__ bool col_sum(double (&v)[NV], double *__restrict__ pa
 // The same for the SpMM kernels, whose threads hold partials for their 4
 // columns: the block's 32 row-lanes per column are folded in (warp, row)
 // order.
-template <int NV>
+template <int NV, bool SPLIT>
 __device__ __forceinline__ bool col_sum4(const double (&v)[NV][kColsPerLane], double (&tot)[NV],
                                          double *__restrict__ partials, unsigned *ticket) {
   __shared__ double part[NV][kCols][kWarps * kRowsPerStep + 1];
   __shared__ double sh[NV][kWarps][kCols];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = warp * kRowsPerStep + (lane >> 3), c0 = (lane & 7) * kColsPerLane;
+  const int slot = warp * kRowsPerStep + (lane >> 3);
+  const Cols<SPLIT> cm{lane & 7};
   const int G = gridDim.x;
 #pragma unroll
   for (int i = 0; i < NV; i++)
 #pragma unroll
-    for (int e = 0; e < kColsPerLane; e++) part[i][c0 + e][slot] = v[i][e];
+    for (int e = 0; e < kColsPerLane; e++) part[i][cm.at(e)][slot] = v[i][e];
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
@@ -273,26 +312,26 @@ __device__ __forceinline__ void update_alldone(MState *ms) {
 }
 
 // R = B - A X, ||b_l||, ||r_l|| (initial state of every column).
-__global__ void __launch_bounds__(kBlock)
-    k_mv_init(SellView<double> a, int apack, const double *__restrict__ X,
+template <int PA, int KA>
+__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+    k_mv_init(InfoView<double> a, const double *__restrict__ X,
               const double *__restrict__ B, double *__restrict__ R, MState *ms,
               double *partials) {
   const int lane = threadIdx.x & 31;
   double pr[2][kColsPerLane] = {};
-  for_each_slice(a, apack, X, [&](int row, int c0, const double (&acc)[kColsPerLane]) {
-    const size_t e0 = (size_t)row * kCols + c0;
+  for_each_slice<PA, KA>(a, X, [&](size_t e0, const auto &cm, const double (&acc)[kColsPerLane]) {
     double b[kColsPerLane], r[kColsPerLane];
-    ldg4(B + e0, b);
+    cm.ldg(B + e0, b);
 #pragma unroll
     for (int e = 0; e < kColsPerLane; e++) {
       r[e] = b[e] - acc[e];
       pr[0][e] += r[e] * r[e];
       pr[1][e] += b[e] * b[e];
     }
-    st4(R + e0, r);
+    cm.st(R + e0, r);
   });
   double tot[2];
-  if (col_sum4<2>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
+  if (col_sum4<2, true>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
     if (lane < ms->m) {
       KState *st = &ms->col[lane];
       const double bn = sqrt(tot[1]);
@@ -305,43 +344,42 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // Sweep 1 of the apply on all columns: T = D^-1 .* (W^T R).
-template <class V, class T>
+template <class V, class T, int PF, int KF>
 __global__ void __launch_bounds__(kBlock, kGatherBlocks)
-    k_mv_sweep1(SellView<V> m, int pack, const double *__restrict__ R, const V *__restrict__ d,
+    k_mv_sweep1(InfoView<V> m, const double *__restrict__ R, const V *__restrict__ d,
                 T *__restrict__ Tm, const MState *ms) {
   if (ms->alldone) return;
   using A = typename Acc<V>::type;
-  for_each_slice(m, pack, R, [&](int row, int c0, const A (&acc)[kColsPerLane]) {
-    const A dr = ldd(d + row);
+  for_each_slice<PF, KF>(m, R, [&](size_t e0, const auto &cm, const A (&acc)[kColsPerLane]) {
+    const A dr = ldd(d + e0 / kCols);
     T t[kColsPerLane];
 #pragma unroll
     for (int e = 0; e < kColsPerLane; e++) t[e] = (T)(dr * acc[e]);
-    st4cs(Tm + (size_t)row * kCols + c0, t);
+    cm.stcs(Tm + e0, t);
   });
 }
 
 // Sweep 2 on all columns: Zv = Z T, with rho_l = r_l . z_l and beta_l.
-template <class V, class T>
+template <class V, class T, int PF, int KF>
 __global__ void __launch_bounds__(kBlock, kGatherBlocks)
-    k_mv_sweep2(SellView<V> m, int pack, const T *__restrict__ Tm, const double *__restrict__ R,
+    k_mv_sweep2(InfoView<V> m, const T *__restrict__ Tm, const double *__restrict__ R,
                 double *__restrict__ Zv, MState *ms, double *partials) {
   if (ms->alldone) return;
   using A = typename Acc<V>::type;
   const int lane = threadIdx.x & 31;
   double pr[1][kColsPerLane] = {};
-  for_each_slice(m, pack, Tm, [&](int row, int c0, const A (&acc)[kColsPerLane]) {
-    const size_t e0 = (size_t)row * kCols + c0;
+  for_each_slice<PF, KF>(m, Tm, [&](size_t e0, const auto &cm, const A (&acc)[kColsPerLane]) {
     double r[kColsPerLane], z[kColsPerLane];
-    ldg4(R + e0, r);
+    cm.ldg(R + e0, r);
 #pragma unroll
     for (int e = 0; e < kColsPerLane; e++) {
       z[e] = (double)acc[e];
       pr[0][e] += r[e] * z[e];
     }
-    st4cs(Zv + e0, z);
+    cm.stcs(Zv + e0, z);
   });
   double tot[1];
-  if (col_sum4<1>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
+  if (col_sum4<1, sizeof(T) == 8>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
     if (lane < ms->m && !ms->col[lane].done) cg_take_rho(&ms->col[lane], tot[0]);
     update_alldone(ms);
   }
@@ -381,22 +419,22 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // Q = A P with sigma_l = p_l . q_l, alpha_l = rho_l / sigma_l.
+template <int PA, int KA>
 __global__ void __launch_bounds__(kBlock, kGatherBlocks)
-    k_mv_spmm_sigma(SellView<double> a, int apack, const double *__restrict__ P,
+    k_mv_spmm_sigma(InfoView<double> a, const double *__restrict__ P,
                     double *__restrict__ Q, MState *ms, double *partials) {
   if (ms->alldone) return;
   const int lane = threadIdx.x & 31;
   double pr[1][kColsPerLane] = {};
-  for_each_slice(a, apack, P, [&](int row, int c0, const double (&acc)[kColsPerLane]) {
-    const size_t e0 = (size_t)row * kCols + c0;
+  for_each_slice<PA, KA>(a, P, [&](size_t e0, const auto &cm, const double (&acc)[kColsPerLane]) {
     double p[kColsPerLane];
-    ldg4(P + e0, p);
+    cm.ldg(P + e0, p);
 #pragma unroll
     for (int e = 0; e < kColsPerLane; e++) pr[0][e] += p[e] * acc[e];
-    st4cs(Q + e0, acc);
+    cm.stcs(Q + e0, acc);
   });
   double tot[1];
-  if (col_sum4<1>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
+  if (col_sum4<1, true>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
     if (lane < ms->m && !ms->col[lane].done) {
       const double p3[3] = {tot[0], 0.0, 0.0};
       finish_dots<kCgSigma>(&ms->col[lane], p3, false, nullptr);
@@ -440,8 +478,9 @@ __device__ __forceinline__ bool col_periodic(const KState &c) {
 
 // Rt = B - A X against R for the columns that need a check; decides
 // confirmation / replacement per column (finish_dots<kTrueRes>).
-__global__ void __launch_bounds__(kBlock)
-    k_mv_trueres(SellView<double> a, int apack, const double *__restrict__ X,
+template <int PA, int KA>
+__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+    k_mv_trueres(InfoView<double> a, const double *__restrict__ X,
                  const double *__restrict__ B, const double *__restrict__ R,
                  double *__restrict__ Rt, MState *ms, double *partials) {
   if (ms->alldone) return;
@@ -451,11 +490,10 @@ __global__ void __launch_bounds__(kBlock)
   const bool verify = lane < ms->m && col_verify(c);
   if (!__syncthreads_or(mine)) return;  // no column needs a check
   double pr[3][kColsPerLane] = {};
-  for_each_slice(a, apack, X, [&](int row, int c0, const double (&acc)[kColsPerLane]) {
-    const size_t e0 = (size_t)row * kCols + c0;
+  for_each_slice<PA, KA>(a, X, [&](size_t e0, const auto &cm, const double (&acc)[kColsPerLane]) {
     double b[kColsPerLane], r[kColsPerLane], rt[kColsPerLane];
-    ldg4(B + e0, b);
-    ldg4(R + e0, r);
+    cm.ldg(B + e0, b);
+    cm.ldg(R + e0, r);
 #pragma unroll
     for (int e = 0; e < kColsPerLane; e++) {
       rt[e] = b[e] - acc[e];
@@ -463,10 +501,10 @@ __global__ void __launch_bounds__(kBlock)
       const double g = rt[e] - r[e];
       pr[1][e] += g * g;
     }
-    st4(Rt + e0, rt);
+    cm.st(Rt + e0, rt);
   });
   double tot[3];
-  if (col_sum4<3>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
+  if (col_sum4<3, true>(pr, tot, partials, &ms->ticket) && threadIdx.x < 32) {
     if (mine) finish_dots<kTrueRes>(&ms->col[lane], tot, verify, nullptr);
     update_alldone(ms);
   }
@@ -574,22 +612,67 @@ int get_ws(ainv_csr *a, MrhsWs **out) {
 }
 
 template <class V, class T>
+struct Sweep1Launch {
+  const MrhsWs *w;
+  const ainv_handle *h;
+  cudaStream_t s;
+  template <int P, int K>
+  void run() const {
+    auto k = k_mv_sweep1<V, T, P, K>;
+    k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(info_view<V>(h->wt), w->v(MR),
+               (const V *)h->d, (T *)w->t, w->st);
+  }
+};
+template <class V, class T>
+struct Sweep2Launch {
+  const MrhsWs *w;
+  const ainv_handle *h;
+  cudaStream_t s;
+  template <int P, int K>
+  void run() const {
+    auto k = k_mv_sweep2<V, T, P, K>;
+    k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(info_view<V>(h->z),
+               (const T *)w->t, w->v(MR), w->v(MZ), w->st, w->partials);
+  }
+};
+template <class V, class T>
 void launch_precond(const MrhsWs *w, const ainv_handle *h, cudaStream_t s) {
-  const SellView<V> wt = view<V>(h->wt), z = view<V>(h->z);
-  const int g1 = wave_grid((const void *)k_mv_sweep1<V, T>, w->n);
-  const int g2 = wave_grid((const void *)k_mv_sweep2<V, T>, w->n);
-  k_mv_sweep1<V, T><<<g1, kBlock, 0, s>>>(wt, h->wt.pack, w->v(MR), (const V *)h->d, (T *)w->t,
-                                         w->st);
-  k_mv_sweep2<V, T><<<g2, kBlock, 0, s>>>(z, h->z.pack, (const T *)w->t, w->v(MR), w->v(MZ),
-                                         w->st, w->partials);
+  with_info<V>(h->wt, Sweep1Launch<V, T>{w, h, s});
+  with_info<V>(h->z, Sweep2Launch<V, T>{w, h, s});
+}
+
+enum Product { kPInit, kPSigma, kPTrueRes };
+struct ProductLaunch {
+  const MrhsWs *w;
+  const DevSell &a;
+  Product what;
+  cudaStream_t s;
+  template <int P, int K>
+  void run() const {
+    const InfoView<double> A = info_view<double>(a);
+    if (what == kPInit) {
+      auto k = k_mv_init<P, K>;
+      k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(A, w->v(MX), w->v(MB),
+                 w->v(MR), w->st, w->partials);
+    } else if (what == kPSigma) {
+      auto k = k_mv_spmm_sigma<P, K>;
+      k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(A, w->v(MP), w->v(MQ),
+                 w->st, w->partials);
+    } else {
+      auto k = k_mv_trueres<P, K>;
+      k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(A, w->v(MX), w->v(MB),
+                 w->v(MR), w->v(MRT), w->st, w->partials);
+    }
+  }
+};
+void launch_product(const MrhsWs *w, const ainv_csr *a, Product what, cudaStream_t s) {
+  with_info<double>(a->a, ProductLaunch{w, a->a, what, s});
 }
 
 int enqueue_iteration(const MrhsWs *w, const ainv_handle *h, const ainv_csr *a) {
   const cudaStream_t s = w->s;
   const long long ne = (long long)w->stride;
-  const SellView<double> A = view<double>(a->a);
   auto gv = [&](const void *k) { return wave_grid(k, ne); };
-  auto gm = [&](const void *k) { return wave_grid(k, w->n); };
   if (h) {
     switch (h->prec) {
       case AINV_PREC_FP64: launch_precond<double, double>(w, h, s); break;
@@ -603,12 +686,10 @@ int enqueue_iteration(const MrhsWs *w, const ainv_handle *h, const ainv_csr *a) 
                                                                w->partials);
   }
   k_mv_p<<<gv((const void *)k_mv_p), kBlock, 0, s>>>(ne, w->v(MZ), w->v(MP), w->st);
-  k_mv_spmm_sigma<<<gm((const void *)k_mv_spmm_sigma), kBlock, 0, s>>>(
-      A, a->a.pack, w->v(MP), w->v(MQ), w->st, w->partials);
+  launch_product(w, a, kPSigma, s);
   k_mv_xr<<<gv((const void *)k_mv_xr), kBlock, 0, s>>>(ne, w->v(MP), w->v(MQ), w->v(MX), w->v(MR),
                                                        w->st, w->partials);
-  k_mv_trueres<<<gm((const void *)k_mv_trueres), kBlock, 0, s>>>(
-      A, a->a.pack, w->v(MX), w->v(MB), w->v(MR), w->v(MRT), w->st, w->partials);
+  launch_product(w, a, kPTrueRes, s);
   k_mv_replace<<<gv((const void *)k_mv_replace), kBlock, 0, s>>>(ne, w->v(MRT), w->v(MR), w->st);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -692,8 +773,7 @@ extern "C" int ainv_gpu_block_solve(ainv_handle *h, const ainv_csr *ac, int m, c
   }
   *w->hst = init;
   AINV_CUDA_TRY(cudaMemcpyAsync(w->st, w->hst, sizeof(MState), cudaMemcpyHostToDevice, w->s));
-  k_mv_init<<<wave_grid((const void *)k_mv_init, n), kBlock, 0, w->s>>>(
-      view<double>(a->a), a->a.pack, w->v(MX), w->v(MB), w->v(MR), w->st, w->partials);
+  launch_product(w, a, kPInit, w->s);
   AINV_CUDA_TRY(cudaGetLastError());
   const bool use_graph = getenv("AINV_NO_GRAPH") == nullptr;
   const long max_chunks = (long)itmax / kChunk + 2 + 4 * kMaxVerifyFails;
