@@ -25,7 +25,7 @@ def dptr(t, n: int, name: str = "vector") -> C.c_void_p:
     call reaches the library."""
     if not (_is_tensor(t) and t.is_cuda):
         raise TypeError(f"{name}: expected a CUDA tensor")
-    if t.dtype != _torch().float64 or not t.is_contiguous():
+    if t.dtype is not _float64() or not t.is_contiguous():
         raise TypeError(f"{name}: expected a contiguous float64 tensor")
     if t.numel() < n:
         raise ValueError(f"{name}: {t.numel()} entries, {n} needed")
@@ -62,9 +62,28 @@ def _torch():
     return torch
 
 
+_F64 = None
+
+
+def _float64():
+    """torch.float64, looked up once: this runs for every vector of a call."""
+    global _F64
+    if _F64 is None:
+        _F64 = _torch().float64
+    return _F64
+
+
+# ctypes form of the trans argument of the usual calls
+_TRANS = {t: t.encode() for t in "NnTtCc"}
+
+
+def _trans(t: str) -> bytes:
+    return _TRANS.get(t) or t.encode()[:1]
+
+
 def _is_tensor(a) -> bool:
     t = type(a)
-    return t.__module__.startswith("torch") and t.__name__ in ("Tensor", "Parameter")
+    return t.__name__ in ("Tensor", "Parameter") and t.__module__.startswith("torch")
 
 
 def _is_cpu_tensor(a) -> bool:
@@ -78,6 +97,7 @@ class DeviceFactors:
         self._own = _borrow is None
         if _borrow is not None:
             self._h = _borrow
+            self._n = None
             return
         self._keep = [_np(wt[0], np.int32), _np(wt[1], np.int32), _np(wt[2], np.float64),
                       _np(z[0], np.int32), _np(z[1], np.int32), _np(z[2], np.float64),
@@ -87,6 +107,7 @@ class DeviceFactors:
         check(lib().ainv_gpu_create(C.byref(h), n, *[C.c_void_p(a.ctypes.data) for a in self._keep],
                                     PREC[prec.upper()], 1 if one_based else 0))
         self._h = h
+        self._n = n  # of a handle of our own, which keeps its size
         del self._keep
 
     @property
@@ -95,7 +116,7 @@ class DeviceFactors:
 
     @property
     def n(self) -> int:
-        return lib().ainv_gpu_get_n(self._h)
+        return lib().ainv_gpu_get_n(self._h) if self._n is None else self._n
 
     @property
     def prec(self) -> str:
@@ -105,8 +126,8 @@ class DeviceFactors:
     def apply(self, x, y, alpha=1.0, beta=0.0, trans="N", stream=None) -> None:
         """y = alpha * Z D^-1 W^T x + beta * y (trans 'N'), device tensors."""
         n = self.n
-        check(lib().ainv_gpu_apply(self._h, trans.encode()[:1], alpha, dptr(x, n, "x"), beta,
-                                   dptr(y, n, "y"), _stream(stream)))
+        check(lib().ainv_gpu_apply(self._h, _trans(trans), alpha, dptr(x, n, "x"), beta,
+                                   dptr(y, n, "y"), None if stream is None else _stream(stream)))
 
     def apply_stage(self, stage, x=None, y=None, alpha=1.0, beta=0.0, trans="N", stream=None):
         """Run sweep 1 (t = D^-1 W^T x) or sweep 2 (y = alpha Z t + beta y) alone."""
@@ -166,7 +187,7 @@ class DeviceFactors:
     def close(self) -> None:
         if getattr(self, "_own", False) and self._h:
             lib().ainv_gpu_destroy(self._h)
-        self._h = None
+        self._h = self._n = None
 
     def __del__(self):
         try:
