@@ -2,6 +2,9 @@
 // PSBLAS psb_dcg / psb_dbicgstab with istop=2 (stop when ||r|| <= eps*||b||),
 // as driven at tests/pdegen/ppde3d.f90:280-281.
 //
+// Small systems run as one persistent kernel (persist.cuh); what follows is
+// the form of the larger ones.  Both give the same iterates.
+//
 // Every scalar of the recurrence (rho, alpha, omega, beta, norms, status)
 // lives in device memory and is produced by the fold kernel that completes
 // the corresponding reduction, so one iteration is a fixed sequence of

@@ -696,17 +696,6 @@ inline void launch_dep(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
 
-// k<<<g, b, smem, s>>>(args...).
-template <class... P, class... A>
-inline void launch(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t s, A &&...a) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = g;
-  cfg.blockDim = b;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
-}
-
 // Blocks for kernels that end in a grid-wide reduction: at most one resident
 // wave (8 blocks of 256 threads per SM) so the last block folds few
 // partials; never more blocks than units of 256 rows.

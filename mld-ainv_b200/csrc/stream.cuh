@@ -1,6 +1,7 @@
-// Streaming sliced SpMV: a persistent kernel feeds shared memory with bulk
-// asynchronous copies (cp.async.bulk, the TMA engine's linear mode) so the
-// bytes in flight do not occupy registers.
+// Streaming sliced SpMV of the solve server's optional operator kernels: a
+// persistent kernel feeds shared memory with bulk asynchronous copies
+// (cp.async.bulk, the TMA engine's linear mode) so the bytes in flight do not
+// occupy registers.
 //
 // Each block walks stages j0, j0 + stride, ... (by default blockIdx.x and
 // gridDim.x; a caller that splits the grid among several vectors passes
@@ -31,10 +32,6 @@ namespace dev {
 
 constexpr int kConsumerWarps = kConsumerSlices;
 constexpr int kStreamThreads = (kConsumerWarps + 1) * 32;  // + the producer warp
-// Blocks a streaming kernel must fit per SM: the register budget of a
-// thread is capped at 65536 / (4 * kStreamThreads) = 56, so that four
-// producers per SM keep their copies in flight.
-constexpr int kStreamMinBlocks = 4;
 // Stage-buffer header: descriptor, then the sptr and iptr chunks (the
 // stage's slice pointers, copied from 16-byte-aligned starts), then the
 // stage's derived words (StageDerived), written by the producer warp.
