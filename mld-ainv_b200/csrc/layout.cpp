@@ -339,30 +339,37 @@ int upload_sell_t(const HostCsr &a, int prec, DevSell &out) {
   idx.resize(idx.size() + 4, 0);  // tail padding: index copies round up to 16 bytes
   sptr.resize(sptr.size() + 4, sptr.back());  // and so do the slice-pointer copies
   iptr.resize(iptr.size() + 4, iptr.back());
-  cudaError_t e = cudaMalloc(&m.sptr, sizeof(int) * sptr.size());
-  if (e == cudaSuccess) e = cudaMalloc(&m.iptr, sizeof(int) * iptr.size());
-  if (e == cudaSuccess && !idx.empty()) e = cudaMalloc(&m.idx, sizeof(int) * idx.size());
-  if (e == cudaSuccess) e = cudaMalloc(&m.info, sizeof(int4) * info.size());
-  if (e == cudaSuccess)
-    e = cudaMemcpy(m.info, info.data(), sizeof(int4) * info.size(), cudaMemcpyHostToDevice);
   pidx.resize(pidx.size() + 4, 0);
-  if (e == cudaSuccess) e = cudaMalloc(&m.pidx, sizeof(int) * pidx.size());
-  if (e == cudaSuccess)
-    e = cudaMemcpy(m.pidx, pidx.data(), sizeof(int) * pidx.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !stages.empty())
-    e = cudaMalloc(&m.stages, sizeof(StageDesc) * stages.size());
-  if (e == cudaSuccess && !stages.empty())
-    e = cudaMemcpy(m.stages, stages.data(), sizeof(StageDesc) * stages.size(),
-                   cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !val.empty()) e = cudaMalloc(&m.val, sizeof(V) * val.size());
-  if (e == cudaSuccess)
-    e = cudaMemcpy(m.sptr, sptr.data(), sizeof(int) * sptr.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(m.iptr, iptr.data(), sizeof(int) * iptr.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !idx.empty())
-    e = cudaMemcpy(m.idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !val.empty())
-    e = cudaMemcpy(m.val, val.data(), sizeof(V) * val.size(), cudaMemcpyHostToDevice);
+  // one allocation for all arrays, 256-byte aligned parts; the word groups come
+  // first, so m.info is its address (free_sell)
+  size_t total = 0;
+  auto part = [&total](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  const size_t o_info = part(sizeof(int4) * info.size());
+  const size_t o_stages = part(sizeof(StageDesc) * stages.size());
+  const size_t o_pidx = part(sizeof(int) * pidx.size());
+  const size_t o_sptr = part(sizeof(int) * sptr.size());
+  const size_t o_iptr = part(sizeof(int) * iptr.size());
+  const size_t o_idx = part(sizeof(int) * idx.size());
+  const size_t o_val = part(sizeof(V) * val.size());
+  char *mem = nullptr;
+  cudaError_t e = cudaMalloc(&mem, total);
+  auto fill = [&](size_t at, const void *src, size_t bytes) -> char * {
+    if (e == cudaSuccess && bytes)
+      e = cudaMemcpy(mem + at, src, bytes, cudaMemcpyHostToDevice);
+    return mem ? mem + at : nullptr;
+  };
+  m.info = reinterpret_cast<int4 *>(fill(o_info, info.data(), sizeof(int4) * info.size()));
+  m.stages = reinterpret_cast<StageDesc *>(
+      fill(o_stages, stages.data(), sizeof(StageDesc) * stages.size()));
+  m.pidx = reinterpret_cast<int *>(fill(o_pidx, pidx.data(), sizeof(int) * pidx.size()));
+  m.sptr = reinterpret_cast<int *>(fill(o_sptr, sptr.data(), sizeof(int) * sptr.size()));
+  m.iptr = reinterpret_cast<int *>(fill(o_iptr, iptr.data(), sizeof(int) * iptr.size()));
+  m.idx = reinterpret_cast<int *>(fill(o_idx, idx.data(), sizeof(int) * idx.size()));
+  m.val = fill(o_val, val.data(), sizeof(V) * val.size());
   if (e != cudaSuccess) {
     free_sell(m);
     set_error("device upload of sliced matrix failed: %s", cudaGetErrorString(e));
@@ -388,13 +395,7 @@ int upload_sell(const HostCsr &a, int prec, DevSell &out) {
 }
 
 void free_sell(DevSell &m) {
-  if (m.stages) cudaFree(m.stages);
-  if (m.info) cudaFree(m.info);
-  if (m.pidx) cudaFree(m.pidx);
-  if (m.sptr) cudaFree(m.sptr);
-  if (m.iptr) cudaFree(m.iptr);
-  if (m.idx) cudaFree(m.idx);
-  if (m.val) cudaFree(m.val);
+  if (m.info) cudaFree(m.info);  // the start of the matrix's allocation
   m = DevSell{};
 }
 
