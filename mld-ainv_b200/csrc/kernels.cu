@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
 // t are computed several times over instead of crossing a grid barrier or a
 // second launch.  The owner also stores its rows of t, as the sweeps do.
 constexpr int kTileBlock = 1024;
+constexpr int kTilePack = 4;  // packs up to which there is such a kernel
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kTileBlock)
     k_apply_tile(InfoView<V> m1, InfoView<V> m2, const double *__restrict__ x,
@@ -290,7 +291,7 @@ struct TileLaunch {
   cudaStream_t s;
   template <int P>
   void run() const {
-    if constexpr (P <= 4)
+    if constexpr (P <= kTilePack)
       launch_dep(k_apply_tile<V, T, P, 4>, (m1.nslices + tile - 1) / tile, kTileBlock,
                  sizeof(T) * kSlice * (size_t)window, s, info_view<V>(m1), info_view<V>(m2), x,
                  (const V *)h->d, (T *)h->t, alpha, beta, y, tile, m2.span);
@@ -391,12 +392,15 @@ constexpr int kTileWindow = 128;
 
 // An apply whose tiles (one per SM) gather few enough rows of t goes out as
 // one launch.  x and y must not overlap: a block reads rows of x that another
-// one owns.
+// one owns.  A BF16 matrix without entries has pack 8 and width 0; it takes
+// the two sweeps.
 static bool apply_tile(const ainv_handle *h, const DevSell &m1, const DevSell &m2, double alpha,
                        const double *x, double beta, double *y, cudaStream_t s) {
   const int tile = (m1.nslices + sm_count() - 1) / sm_count();
   const long long window = (long long)tile + m2.span / kSlice + 1;
-  if (window > kTileWindow || m1.pack != m2.pack || m1.wmax > 4 || m2.wmax > 4) return false;
+  if (window > kTileWindow || m1.pack != m2.pack || m1.pack > kTilePack || m1.wmax > 4 ||
+      m2.wmax > 4)
+    return false;
   const uintptr_t xa = (uintptr_t)x, ya = (uintptr_t)y, nb = sizeof(double) * (uintptr_t)h->n;
   if (xa < ya + nb && ya < xa + nb) return false;
   by_prec(m1.prec, [&](auto ty) {
