@@ -34,10 +34,10 @@ using namespace dev;
 // sweep 2 389 MB in 60.7 us, 6.4 TB/s each.
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
-    k_sweep_dscale(InfoView<V> m, const double *__restrict__ x, const V *__restrict__ d,
-                   T *__restrict__ t, int s0, int s1, const int *__restrict__ stop) {
+    k_sweep_dscale(InfoView<V> m, const double *x, const V *d, T *t, int s0, int s1,
+                   const volatile int *stop) {
   for_each_info<P, K>(
-      m, x, s0, s1, [&] { return !stop || !*stop; }, [&](int row) { return ldd(d + row); },
+      m, x, s0, s1, [&] { return !stop || !*stop; }, [&](int row) { return ldd_now(d + row); },
       [&](int row, auto acc, auto dr) { t[row] = (T)(dr * acc); }, [](int) {});
 }
 
@@ -45,11 +45,11 @@ __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
 // axpby_row, so all forms give the same bits.
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
-    k_sweep_axpby(InfoView<V> m, const T *__restrict__ t, double alpha, double beta,
-                  double *__restrict__ y, int s0, int s1, const int *__restrict__ stop) {
+    k_sweep_axpby(InfoView<V> m, const T *t, double alpha, double beta, double *y, int s0, int s1,
+                  const volatile int *stop) {
   for_each_info<P, K>(
       m, t, s0, s1, [&] { return !stop || !*stop; },
-      [&](int row) { return beta == 0.0 ? 0.0 : y[row]; },
+      [&](int row) { return beta == 0.0 ? 0.0 : ld_now(y + row); },
       [&](int row, auto acc, double yr) { y[row] = axpby_row(alpha, (double)acc, beta, yr); },
       [](int) {});
 }
@@ -64,9 +64,8 @@ constexpr int kTileBlock = 1024;
 constexpr int kTilePack = 4;  // packs up to which there is such a kernel
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kTileBlock)
-    k_apply_tile(InfoView<V> m1, InfoView<V> m2, const double *__restrict__ x,
-                 const V *__restrict__ d, T *__restrict__ t, double alpha, double beta,
-                 double *__restrict__ y, int tile, int span) {
+    k_apply_tile(InfoView<V> m1, InfoView<V> m2, const double *x, const V *d, T *t, double alpha,
+                 double beta, double *y, int tile, int span) {
   using A = typename Acc<V>::type;
   constexpr int kStep = kTileBlock / 32;
   extern __shared__ __align__(16) unsigned char tile_smem[];
@@ -81,10 +80,10 @@ __global__ void __launch_bounds__(kTileBlock)
   if (a + warp < we) f = __ldg(m1.info + a + warp);
   info_load(m1, f, 0, b);
   dep_wait();
-  const auto gx = [&](int c) { return (unsigned)c < (unsigned)m1.n ? __ldg(x + c) : 0.0; };
+  const auto gx = [&](int c) { return (unsigned)c < (unsigned)m1.n ? ld_now(x + c) : 0.0; };
   for (int s = a + warp; s < we; s += kStep) {
     const int row = s * kSlice + lane;
-    const A dr = ldd(d + min(row, m1.n - 1));
+    const A dr = ldd_now(d + min(row, m1.n - 1));
     int4 fn = f;
     if (s + kStep < we) fn = __ldg(m1.info + s + kStep);
     A acc = A(0);
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(kTileBlock)
       f = __ldg(m2.info + q);
       info_load(m2, f, 0, b);
     }
-    const double yr = beta == 0.0 ? 0.0 : y[min(row, m2.n - 1)];
+    const double yr = beta == 0.0 ? 0.0 : ld_now(y + min(row, m2.n - 1));
     A acc = A(0);
     info_sum<T>(b, f.w ? row : 0, gt, acc);
     for (int k0 = K; k0 < f.z; k0 += K) {

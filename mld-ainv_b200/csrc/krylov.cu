@@ -75,8 +75,7 @@ struct SliceOut {
 // reduction that did not run is not folded.
 template <int NV, class Fin>
 __global__ void __launch_bounds__(kFoldThreads)
-    k_fold(const double *__restrict__ sp, int ld, int ns, int ng, double *__restrict__ rs,
-           int ldr, KState *st, Fin fin) {
+    k_fold(const double *sp, int ld, int ns, int ng, double *rs, int ldr, KState *st, Fin fin) {
   dep_start();
   dep_wait();
   if (fin.skip(st)) return;
@@ -163,7 +162,7 @@ __device__ __forceinline__ int nslices_of(int n) { return (n + kSlice - 1) / kSl
 
 // ||b||_2 (istop=2 denominator).
 __global__ void __launch_bounds__(kBlock)
-    k_bnorm(int n, const double *__restrict__ b, SliceOut o) {
+    k_bnorm(int n, const double *b, SliceOut o) {
   dep_start();
   dep_wait();
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
@@ -183,9 +182,8 @@ __device__ __forceinline__ bool dots_skip(const KState *st) {
 
 template <int MODE, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<double, K>())
-    k_spmv_dots(InfoView<double> m, const double *__restrict__ x, double *__restrict__ y,
-                const double *__restrict__ w1, double *__restrict__ w2,
-                const double *__restrict__ w3, const KState *st, SliceOut o) {
+    k_spmv_dots(InfoView<double> m, const double *x, double *y, const double *w1, double *w2,
+                const double *w3, const KState *st, SliceOut o) {
   SliceSums<dots_of(MODE)> ss{o.sp, o.ld, {}};
   const double *a = dots_operand<MODE>(x, w1);
   for_each_info<P, K>(
@@ -196,8 +194,7 @@ __global__ void __launch_bounds__(kBlock, info_blocks<double, K>())
 
 // r := b - A x when the last true-residual check asked for it.
 __global__ void __launch_bounds__(kBlock)
-    k_replace_r(int n, const double *__restrict__ rtrue, double *__restrict__ r,
-                const KState *st) {
+    k_replace_r(int n, const double *rtrue, double *r, const KState *st) {
   dep_start();
   dep_wait();
   if (!st->replace) return;
@@ -207,8 +204,8 @@ __global__ void __launch_bounds__(kBlock)
 // CG: z = Z t (sweep 2 of the AINV apply) fused with rho = r.z.
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
-    k_cg_sweep2(InfoView<V> m, const T *__restrict__ t, const double *__restrict__ r,
-                double *__restrict__ z, const KState *st, SliceOut o) {
+    k_cg_sweep2(InfoView<V> m, const T *t, const double *r, double *z, const KState *st,
+                SliceOut o) {
   SliceSums<1> ss{o.sp, o.ld, {0.0}};
   for_each_info<P, K>(
       m, t, 0, m.nslices, [&] { return !st->done; }, [&](int i) { return r[i]; },
@@ -222,8 +219,7 @@ __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
 
 // CG without preconditioner: z = r, rho = r.r.
 __global__ void __launch_bounds__(kBlock)
-    k_cg_ident(int n, const double *__restrict__ r, double *__restrict__ z, const KState *st,
-               SliceOut o) {
+    k_cg_ident(int n, const double *r, double *z, const KState *st, SliceOut o) {
   dep_start();
   dep_wait();
   if (st->done) return;
@@ -241,7 +237,7 @@ __global__ void __launch_bounds__(kBlock)
 
 // CG: p = z (first iteration) or p = z + beta p.
 __global__ void __launch_bounds__(kBlock)
-    k_cg_p(int n, const double *__restrict__ z, double *__restrict__ p, const KState *st) {
+    k_cg_p(int n, const double *z, double *p, const KState *st) {
   dep_start();
   dep_wait();
   if (st->done) return;
@@ -252,8 +248,8 @@ __global__ void __launch_bounds__(kBlock)
 
 // CG: x += alpha p, r -= alpha q, rn2 = r.r.
 __global__ void __launch_bounds__(kBlock)
-    k_cg_xr(int n, const double *__restrict__ p, const double *__restrict__ q,
-            double *__restrict__ x, double *__restrict__ r, const KState *st, SliceOut o) {
+    k_cg_xr(int n, const double *p, const double *q, double *x, double *r, const KState *st,
+            SliceOut o) {
   dep_start();
   dep_wait();
   if (st->done) return;
@@ -274,8 +270,7 @@ __global__ void __launch_bounds__(kBlock)
 
 // BiCGSTAB: p = r (first iteration) or p = r + beta (p - omega v).
 __global__ void __launch_bounds__(kBlock)
-    k_bicg_p(int n, const double *__restrict__ r, const double *__restrict__ v,
-             double *__restrict__ p, const KState *st) {
+    k_bicg_p(int n, const double *r, const double *v, double *p, const KState *st) {
   dep_start();
   dep_wait();
   if (st->done) return;
@@ -286,8 +281,7 @@ __global__ void __launch_bounds__(kBlock)
 
 // BiCGSTAB: s = r - alpha v.
 __global__ void __launch_bounds__(kBlock)
-    k_bicg_s(int n, const double *__restrict__ r, const double *__restrict__ v,
-             double *__restrict__ s, const KState *st) {
+    k_bicg_s(int n, const double *r, const double *v, double *s, const KState *st) {
   dep_start();
   dep_wait();
   if (st->done) return;
@@ -298,10 +292,8 @@ __global__ void __launch_bounds__(kBlock)
 
 // BiCGSTAB: x += alpha f + omega z, r = s - omega t, rn2 = r.r, rho' = rt.r.
 __global__ void __launch_bounds__(kBlock)
-    k_bicg_xr(int n, const double *__restrict__ f, const double *__restrict__ z,
-              const double *__restrict__ s, const double *__restrict__ t,
-              const double *__restrict__ rt, double *__restrict__ x,
-              double *__restrict__ r, const KState *st, SliceOut o) {
+    k_bicg_xr(int n, const double *f, const double *z, const double *s, const double *t,
+              const double *rt, double *x, double *r, const KState *st, SliceOut o) {
   dep_start();
   dep_wait();
   if (st->done) return;

@@ -232,20 +232,7 @@ __device__ __forceinline__ typename Acc<V>::type slab_dot(const PMat<V> &a,
 }
 
 // ---- gathered vectors ---------------------------------------------------------
-// These vectors are written while the kernel runs, so their loads are coherent
-// ones that the compiler must not move across a barrier or reuse after one:
-// volatile (the __ldca and __ldcg intrinsics are functions of the address
-// alone to it).
-__device__ __forceinline__ double ld_now(const double *p) {
-  double v;
-  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ float ld_now(const float *p) {
-  float v;
-  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
+// These vectors are written while the kernel runs: ordinary, volatile loads.
 template <class X>
 struct GVec {
   static constexpr int kBatch = 8;

@@ -31,12 +31,38 @@ __device__ __forceinline__ float ldv(const __nv_bfloat16 *p) {
   unsigned short u = __ldcs(reinterpret_cast<const unsigned short *>(p));
   return __uint_as_float(((unsigned)u) << 16);
 }
-// Cached loads for per-row vectors (D^-1).
+// Cached loads for per-row vectors (D^-1), through the read-only path.
 __device__ __forceinline__ double ldd(const double *p) { return __ldg(p); }
 __device__ __forceinline__ float ldd(const float *p) { return __ldg(p); }
 __device__ __forceinline__ float ldd(const __nv_bfloat16 *p) {
   unsigned short u = __ldg(reinterpret_cast<const unsigned short *>(p));
   return __uint_as_float(((unsigned)u) << 16);
+}
+
+// Loads of memory that other kernels, or other blocks of this one, write while
+// the kernel is resident: ordinary ones that the compiler must not move across
+// a wait or reuse after one, so volatile (the __ldca and __ldcg intrinsics are
+// functions of the address alone to it).
+__device__ __forceinline__ double ld_now(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_now(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_now(const unsigned short *p) {
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+// The same for D^-1 (ldd).
+__device__ __forceinline__ double ldd_now(const double *p) { return ld_now(p); }
+__device__ __forceinline__ float ldd_now(const float *p) { return ld_now(p); }
+__device__ __forceinline__ float ldd_now(const __nv_bfloat16 *p) {
+  return __uint_as_float(ld_now(reinterpret_cast<const unsigned short *>(p)) << 16);
 }
 
 // c + a*b of the row accumulations.  In FP64 the product and the sum each
@@ -83,6 +109,10 @@ __device__ __forceinline__ double ldv(const b16w *p) {
 __device__ __forceinline__ double ldd(const f32w *p) { return (double)__ldg(&p->v); }
 __device__ __forceinline__ double ldd(const b16w *p) {
   return (double)__uint_as_float(((unsigned)__ldg(&p->v)) << 16);
+}
+__device__ __forceinline__ double ldd_now(const f32w *p) { return (double)ld_now(&p->v); }
+__device__ __forceinline__ double ldd_now(const b16w *p) {
+  return (double)__uint_as_float(ld_now(&p->v) << 16);
 }
 template <class V>
 constexpr bool is_acc64() { return std::is_same<V, f32w>::value || std::is_same<V, b16w>::value; }
@@ -438,7 +468,11 @@ inline InfoView<V> info_view(const DevSell &m) {
 // touches nothing but matrix words, which no kernel writes (D^-1 is not among
 // them: update_a writes it).  Every block waits, so a grid ends after the one
 // before it whatever its blocks do; dep_start lets the next grid's blocks in
-// as this one's leave.
+// as this one's leave.  What other kernels write (vectors, D^-1, sums, flags)
+// is therefore not constant while such a kernel is resident, and several of
+// them are resident together: it is read with ordinary loads (ld_now; no
+// __ldg, and no __restrict__ pointer to it), never through the read-only path,
+// which may keep lines that an older grid brought in.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -450,7 +484,7 @@ __device__ __forceinline__ void dep_start() {
 // are those of group_slots, in the same order.
 template <int P, int K, class V, class X>
 __device__ __forceinline__ typename Acc<V>::type info_dot(const InfoView<V> &m, const int4 &f,
-                                                          int row, const X *__restrict__ x) {
+                                                          int row, const X *x) {
   using A = typename Acc<V>::type;
   static_assert(K % P == 0, "whole packs");
   constexpr int J = K / P;
@@ -481,7 +515,7 @@ __device__ __forceinline__ typename Acc<V>::type info_dot(const InfoView<V> &m, 
 #pragma unroll
         for (int e = 0; e < P; e++) {
           const int col = row + c[j][e];
-          xv[j][e] = (unsigned)col < (unsigned)m.n ? __ldg(x + col) : X(0);
+          xv[j][e] = (unsigned)col < (unsigned)m.n ? ld_now(x + col) : X(0);
         }
 #pragma unroll
       for (int j = 0; j < J; j++)
@@ -513,7 +547,7 @@ __device__ __forceinline__ typename Acc<V>::type info_dot(const InfoView<V> &m, 
       for (int j = 0; j < J; j++)
 #pragma unroll
         for (int e = 0; e < P; e++)
-          xv[j][e] = (unsigned)c[j][e] < (unsigned)m.n ? __ldg(x + c[j][e]) : X(0);
+          xv[j][e] = (unsigned)c[j][e] < (unsigned)m.n ? ld_now(x + c[j][e]) : X(0);
 #pragma unroll
       for (int j = 0; j < J; j++)
 #pragma unroll
@@ -609,7 +643,7 @@ inline bool with_info(const DevSell &m, const F &f) {
 // and end(s) with the whole warp.  The first slice's words are loaded before
 // dep_wait; go() decides after it whether there is anything to do.
 template <int P, int K, class V, class X, class Go, class Pre, class Post, class End>
-__device__ __forceinline__ void for_each_info(const InfoView<V> &m, const X *__restrict__ x,
+__device__ __forceinline__ void for_each_info(const InfoView<V> &m, const X *x,
                                               int s0, int s1, Go &&go, Pre &&pre, Post &&post,
                                               End &&end) {
   using A = typename Acc<V>::type;
@@ -741,7 +775,7 @@ __device__ __forceinline__ void block_sum(double (&v)[NV]) {
 // loaded before the first add), then block_sum folds the block's groups.
 // The range sums are valid in thread 0.
 template <int NV>
-__device__ __forceinline__ void fold_range(const double *__restrict__ sp, int ld, int ns, int ng,
+__device__ __forceinline__ void fold_range(const double *sp, int ld, int ns, int ng,
                                            int r, double (&v)[NV]) {
   static_assert(kFoldRange == kFoldThreads, "one group per thread");
   const int g0 = r * kFoldRange, g1 = min(ng, g0 + kFoldRange);
@@ -752,7 +786,7 @@ __device__ __forceinline__ void fold_range(const double *__restrict__ sp, int ld
 #pragma unroll
     for (int j = 0; j < kGroupSlices; j++) {
       const int sl = g * kGroupSlices + j;
-      raw[k][j] = (g < g1 && sl < ns) ? __ldg(sp + (size_t)k * ld + sl) : 0.0;
+      raw[k][j] = (g < g1 && sl < ns) ? ld_now(sp + (size_t)k * ld + sl) : 0.0;
     }
 #pragma unroll
   for (int k = 0; k < NV; k++) {
