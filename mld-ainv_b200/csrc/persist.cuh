@@ -595,6 +595,7 @@ struct PLoop {
             if (!sync()) return false;
             continue;
           }
+          __syncthreads();  // all have read done, which thread 0 may set now
           if (threadIdx.x == 0) kstate::cg_take_rho(&sh.k, sh.rho);
           __syncthreads();
         } else if (last) {
