@@ -189,6 +189,9 @@ bool host_pipe_usable(const ainv_handle *h, bool tr, const double *y);
 int host_pipe_apply(ainv_handle *h, bool tr, const HostPlan &p, double alpha, const double *x,
                     double beta, double *y, cudaStream_t si, cudaStream_t sc);
 int host_pipe_status(const ainv_handle *h);
+// Limit of a wait of the persistent Krylov loop in microseconds: 2 s, or
+// AINV_WAIT_MS milliseconds when that is set.
+unsigned wait_limit_us();
 void destroy_host_pipe(HostPipe *hp);
 }  // namespace ainv
 

@@ -56,7 +56,7 @@ constexpr int kChunk = 10;
 static_assert(kRecheck % kChunk == 0, "periodic checks fall on chunk ends");
 constexpr int kHistCap = 8192;  // iterations whose residual is recorded
 // Arrival counters of the persistent loop, on cache lines of their own.
-constexpr int kBarLine = 32, kBarWords = 3 * kBarLine;
+constexpr int kBarLine = 32, kBarWords = 2 * kBarLine;
 constexpr int kPersistIters = 1024;  // iterations per launch of it
 
 // Where a reduction kernel stores its sums: dot k of group g (or of slice
@@ -365,7 +365,19 @@ void spmv_dots(const DevSell &A, cudaStream_t s, const double *x, double *y, con
 
 std::atomic<unsigned long long> g_serial{1};
 
+// What the host reads of a loop: its state, and the persistent loop's abort word.
+struct LoopState {
+  KState k;
+  int abort;
+};
+
 }  // namespace
+
+unsigned wait_limit_us() {
+  const char *e = std::getenv("AINV_WAIT_MS");
+  const long long ms = e ? std::atoll(e) : 2000;
+  return (unsigned)(std::min(std::max(ms, 0ll), 1000000ll) * 1000);
+}
 
 unsigned long long next_serial() { return g_serial.fetch_add(1); }
 
@@ -384,11 +396,13 @@ struct KrylovWs {
   double *hist_h = nullptr;  // page-locked
   std::vector<double> hhist;
   int hcount = 0;
-  // persistent loop: two arrival counters used in turn, and the abort word
+  // persistent loop: two arrival counters used in turn
   unsigned *bar = nullptr;
   unsigned turn = 0;
-  KState *st = nullptr;
-  KState *hst = nullptr;  // pinned mirror
+  LoopState *loop = nullptr;
+  KState *st = nullptr;       // &loop->k
+  LoopState *hloop = nullptr;  // page-locked mirror
+  KState *hst = nullptr;      // &hloop->k
   cudaStream_t s = nullptr;
   cudaEvent_t ev = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -447,7 +461,7 @@ int get_ws(ainv_csr *a, KrylovWs **out) {
   const size_t sp = part(sizeof(double) * 3 * (size_t)w->ld);
   const size_t rs = part(sizeof(double) * 3 * (size_t)w->ldr);
   const size_t hist = part(sizeof(double) * kHistCap);
-  const size_t bar = part(sizeof(unsigned) * kBarWords), st = part(sizeof(KState));
+  const size_t bar = part(sizeof(unsigned) * kBarWords), loop = part(sizeof(LoopState));
   cudaError_t e = cudaMalloc(&w->mem, at);
   if (e == cudaSuccess) e = cudaMemset(w->mem, 0, at);
   w->vec = reinterpret_cast<double *>(w->mem + vec);
@@ -455,10 +469,12 @@ int get_ws(ainv_csr *a, KrylovWs **out) {
   w->rs = reinterpret_cast<double *>(w->mem + rs);
   w->hist = reinterpret_cast<double *>(w->mem + hist);
   w->bar = reinterpret_cast<unsigned *>(w->mem + bar);
-  w->st = reinterpret_cast<KState *>(w->mem + st);
-  const size_t hh = (sizeof(KState) + 255) / 256 * 256;
+  w->loop = reinterpret_cast<LoopState *>(w->mem + loop);
+  w->st = &w->loop->k;
+  const size_t hh = (sizeof(LoopState) + 255) / 256 * 256;
   if (e == cudaSuccess) e = cudaMallocHost(&w->hmem, hh + sizeof(double) * kHistCap);
-  w->hst = reinterpret_cast<KState *>(w->hmem);
+  w->hloop = reinterpret_cast<LoopState *>(w->hmem);
+  w->hst = &w->hloop->k;
   w->hist_h = reinterpret_cast<double *>(w->hmem + hh);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev, cudaEventDisableTiming);
@@ -636,7 +652,8 @@ int persist_launch_mb(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, cons
   p.ng = w->ng;
   p.bar = w->bar + (w->turn & 1u) * kBarLine;
   p.bar_next = w->bar + ((w->turn + 1) & 1u) * kBarLine;
-  p.abort = reinterpret_cast<int *>(w->bar + 2 * kBarLine);
+  p.abort = &w->loop->abort;
+  p.wait_us = wait_limit_us();
   p.st = w->st;
   p.resume = resume;
   p.max_iters = kPersistIters;
@@ -744,8 +761,8 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   init.method = method;
   init.hist = w->hist;
   init.hist_cap = kHistCap;
-  *w->hst = init;
-  AINV_CUDA_TRY(cudaMemcpyAsync(w->st, w->hst, sizeof(KState), cudaMemcpyHostToDevice, w->s));
+  *w->hloop = LoopState{init, 0};
+  AINV_CUDA_TRY(cudaMemcpyAsync(w->loop, w->hloop, sizeof(LoopState), cudaMemcpyHostToDevice, w->s));
   const bool persistent =
       h && n <= kPMaxRows && w->ng <= kPMaxPerTeam * kPTeams * 2 * sm_count();
   if (persistent) {
@@ -753,13 +770,16 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
       const int rc = persist(w, h, a, b, x, method, resume);
       if (rc == AINV_ERR_UNSUPPORTED && !resume) break;  // no cooperative launch: plain loop
       AINV_TRY(rc);
-      AINV_CUDA_TRY(cudaMemcpyAsync(w->hst, w->st, sizeof(KState), cudaMemcpyDeviceToHost, w->s));
+      AINV_CUDA_TRY(cudaMemcpyAsync(w->hloop, w->loop, sizeof(LoopState), cudaMemcpyDeviceToHost,
+                                    w->s));
       AINV_CUDA_TRY(cudaMemcpyAsync(w->hist_h, w->hist,
                                     sizeof(double) * (size_t)std::min(itmax, kHistCap),
                                     cudaMemcpyDeviceToHost, w->s));
       AINV_CUDA_TRY(cudaStreamSynchronize(w->s));
-      if (w->hst->timeout)
+      if (w->hloop->abort) {
+        w->hst->timeout = 1;
         AINV_CUDA_TRY(cudaMemset(w->bar, 0, sizeof(unsigned) * kBarWords));
+      }
       if (w->hst->done || w->hst->timeout) {
         AINV_CUDA_TRY(cudaEventRecord(w->ev, w->s));
         AINV_CUDA_TRY(cudaStreamWaitEvent(user, w->ev, 0));

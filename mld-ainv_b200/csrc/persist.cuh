@@ -33,8 +33,10 @@
 // the three matrices in them (12.4 -> 11.0 us per CG iteration at 40^3);
 // above that, two blocks per SM with 64 registers read them in each phase.
 //
-// Every wait is bounded (kWaitNs); a block that gives up sets the abort word,
-// which ends the others' waits, and the state's timeout flag.
+// Every wait is bounded (wait_limit_us); a block that gives up sets the abort
+// word, which ends the others' waits.  Other blocks, the one that stores the
+// state among them, may still pass their last barrier, so the abort word goes
+// to the host with the state and decides whether the loop timed out.
 #pragma once
 
 #include "krylov_epi.cuh"
@@ -83,7 +85,8 @@ struct PArgs {
   double *gs;               // group sums: kPBufs buffers of 3 x ng
   int n, ns, ng;
   unsigned *bar, *bar_next;  // this launch's arrival counter; the next one's, cleared here
-  int *abort;
+  int *abort;        // 0 at the launch; set by a block that gives up
+  unsigned wait_us;  // limit of a wait; 0: any wait is given up
   KState *st;
   int resume;     // continue from *st
   int max_iters;  // iterations of this launch at most
@@ -116,7 +119,7 @@ struct GridBarrier {
   unsigned nb, target;
   // Called by every thread of the block; false once a wait was given up
   // (by any block).
-  __device__ __forceinline__ bool wait(PShared &sh) {
+  __device__ __forceinline__ bool wait(PShared &sh, unsigned wait_us) {
     // The block's writes reach the other blocks by the release of thread 0
     // (the block barrier orders them before it), theirs this block by its
     // acquire.
@@ -128,8 +131,9 @@ struct GridBarrier {
         const unsigned long long t0 = global_ns();
         for (unsigned it = 1;; ++it) {
           if (ld_acquire(ctr) >= target) break;
-          if ((it & 63u) == 0 &&
-              (*(volatile int *)abort != 0 || global_ns() - t0 > kWaitNs || it > (1u << 30))) {
+          if (((it & 63u) == 0 || wait_us == 0) &&
+              (*(volatile int *)abort != 0 || global_ns() - t0 >= wait_us * 1000ull ||
+               it > (1u << 30))) {
             *(volatile int *)abort = 1;
             sh.dead = 1;
             break;
@@ -397,7 +401,7 @@ struct PLoop {
     for (int k = 0; k < NV; k++) src[k] = sums + (size_t)k * a.ng;
     fold_groups<NV>(src, a.ng, sh, fin);
   }
-  __device__ __forceinline__ bool sync() { return bar.wait(sh); }
+  __device__ __forceinline__ bool sync() { return bar.wait(sh, a.wait_us); }
   template <int NV, class Body>
   __device__ __forceinline__ void groups(Body &&body) {
     for_groups<NV>(a.n, a.ns, a.ng, lb, nb, sh, gs(), body);

@@ -149,7 +149,8 @@ struct Table {
 struct SlotState {
   KState k;
   int phase;
-  int pad[3];
+  int abort;  // persistent loop: a block of the slot gave up a wait
+  int pad[2];
 };
 
 inline Mat mat_of(const DevSell &m) {
@@ -894,11 +895,11 @@ constexpr int kPersistBlocks = 2;  // per SM
 // 16.7, 16 of 64^3 (27.7) 26.7 / 27.3; past that the two are level, and the
 // batched kernels share an operator's reads.
 constexpr int kPersistPerTeam = 32;
-// Arrival counters and abort words: [parity][slot], on lines of their own.
+// Arrival counters: [parity][slot], on lines of their own.
 constexpr int kBarLine = 32;
-constexpr int kBarWords = 2 * 2 * kMaxSlots * kBarLine;
-__device__ __forceinline__ unsigned *bar_word(unsigned *bars, int what, int parity, int slot) {
-  return bars + ((what * 2 + parity) * kMaxSlots + slot) * kBarLine;
+constexpr int kBarWords = 2 * kMaxSlots * kBarLine;
+__device__ __forceinline__ unsigned *bar_word(unsigned *bars, int parity, int slot) {
+  return bars + (parity * kMaxSlots + slot) * kBarLine;
 }
 
 template <class V>
@@ -908,14 +909,12 @@ __device__ __forceinline__ PMat<V> pmat_of(const Mat &m) {
 
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kPBlock, kPersistBlocks)
-    k_srv_persist(const Table *tab, SlotState *sts, unsigned *bars, int parity, int iters) {
+    k_srv_persist(const Table *tab, SlotState *sts, unsigned *bars, int parity, int iters,
+                  unsigned wait_us) {
   __shared__ PShared sh;
   __shared__ PArgs<V, T> a;
-  // the words of the next launch, for every slot
-  if (blockIdx.x == 0 && threadIdx.x < kMaxSlots) {
-    *bar_word(bars, 0, parity ^ 1, threadIdx.x) = 0u;
-    *bar_word(bars, 1, parity ^ 1, threadIdx.x) = 0u;
-  }
+  // the counters of the next launch, for every slot
+  if (blockIdx.x == 0 && threadIdx.x < kMaxSlots) *bar_word(bars, parity ^ 1, threadIdx.x) = 0u;
   const int slot = tab->block_slot_p[blockIdx.x];
   if (slot < 0) return;
   SlotState *ss = sts + slot;
@@ -938,8 +937,9 @@ __global__ void __launch_bounds__(kPBlock, kPersistBlocks)
     a.n = sd.n;
     a.ns = sd.ns;
     a.ng = sd.ng;
-    a.bar = bar_word(bars, 0, parity, slot);
-    a.abort = (int *)bar_word(bars, 1, parity, slot);
+    a.bar = bar_word(bars, parity, slot);
+    a.abort = &ss->abort;
+    a.wait_us = wait_us;
     a.max_iters = iters;
   }
   __syncthreads();
@@ -1304,7 +1304,8 @@ struct ainv_server {
   ainv::srv::LaunchPlan plan, graph_plan;   // launches the operators need / in the graph
   int graph_kernels = 0;                    // kernel launches per graph launch
   ainv::srv::SlotState *st_d = nullptr, *st_h = nullptr;
-  unsigned *bars = nullptr;      // persistent loop: arrival counters and abort words
+  unsigned *bars = nullptr;      // persistent loop: arrival counters
+  unsigned wait_us = 0;          // and the limit of its waits
   int parity = 0;                // which of them the next launch uses
   void *persist = nullptr;       // kernel for the admitted mix, or null: the graph
   char *arena_d = nullptr;
@@ -1537,7 +1538,7 @@ void plan_persist(ainv_server *srv, const std::vector<int> &order) {
 // the mix changes) if the device does not take the grid at once.
 bool launch_persist(ainv_server *srv) {
   int iters = srv->iters;
-  void *args[] = {&srv->tab_d, &srv->st_d, &srv->bars, &srv->parity, &iters};
+  void *args[] = {&srv->tab_d, &srv->st_d, &srv->bars, &srv->parity, &iters, &srv->wait_us};
   const int grid = std::min(kMaxGrid, kPersistBlocks * sm_count());
   if (cudaLaunchCooperativeKernel(srv->persist, dim3(grid), dim3(kPBlock), args, 0, srv->s) !=
       cudaSuccess) {
@@ -1699,7 +1700,8 @@ void engine_loop(ainv_server *srv) {
     std::vector<int> done;
     for (int k = 0; k < S; k++) {
       const SlotHost &sl = srv->slots[(size_t)k];
-      // finished, or a streamed kernel gave up a bounded wait for it
+      // finished, or a kernel gave up a bounded wait for it
+      if (srv->st_h[k].abort) srv->st_h[k].k.timeout = 1;
       if (sl.req && ((srv->st_h[k].phase == kRun && srv->st_h[k].k.done) || srv->st_h[k].k.timeout)) {
         done.push_back(k);
         ENG_TRY(cudaMemcpyAsync(sl.req->x, srv->tab_h->slot[k].vec[VX],
@@ -1772,6 +1774,7 @@ int ainv_server_create(ainv_server **out, int max_slots, size_t hbm_bytes, int i
   }
   srv->max_slots = max_slots;
   srv->iters = iters_per_launch;
+  srv->wait_us = ainv::wait_limit_us();
   srv->slots.resize((size_t)max_slots);
   srv->t0 = std::chrono::steady_clock::now();
   auto fail = [&](cudaError_t e, const char *what) {
@@ -1944,6 +1947,9 @@ int ainv_server_wait(ainv_server *srv, long long id, double timeout_s, ainv_resu
       case AINV_ERR_NOCONV: ainv::set_error("request %lld: itmax reached", id); break;
       case AINV_ERR_BREAKDOWN: ainv::set_error("request %lld: Krylov breakdown", id); break;
       case AINV_ERR_NONFINITE: ainv::set_error("request %lld: non-finite residual", id); break;
+      case AINV_ERR_TIMEOUT:
+        ainv::set_error("request %lld: a device wait ran past its time limit", id);
+        break;
       default: ainv::set_error("request %lld: %s", id, srv->error_msg.c_str()); break;
     }
   }
