@@ -36,14 +36,18 @@ using namespace kstate;
 constexpr int kCols = 32;    // multivector stride (columns per row)
 constexpr int kChunk = 8;    // iterations per captured graph launch
 constexpr int kRecheck = 50; // true-residual period for FP32/BF16 factors
-// Resident blocks per SM asked of the gathering kernels (SpMM and sweeps):
-// 4 (64 registers) measured 0.489 s per 128^3 x 32 block solve, 5 (48
-// registers, a few spills) 0.500 s, 6 (40) and an uncapped build (72-96
-// registers) 0.54 s.
-#ifndef AINV_MRHS_BLOCKS
-#define AINV_MRHS_BLOCKS 4
-#endif
-constexpr int kGatherBlocks = AINV_MRHS_BLOCKS;
+// Resident blocks per SM asked of the gathering kernels.  Products with A: 2;
+// at 4 (64 registers) the slab, the gathers and the sums of 8 slots spill 124
+// to 284 bytes.  us per iteration with 32 right-hand sides at 4 / 2: FP64
+// factors of 4 slots 24^3 94 / 86, 64^3 326 / 319, 100^3 1007 / 951; FP32 88 /
+// 81, 298 / 291, 892 / 833; INVK(1,1) FP64 182 / 172, 573 / 562, 1920 / 1866;
+// 27-point A 64^3 435 / 447, 90^3 1037 / 1034.  Sweeps: 4.  Those of more than 4
+// slots, and sweep 2 of 4 slots, spill up to 180 bytes where they sum in FP64,
+// and warps are worth it: with 3 blocks 64^3 INVK FP64 takes 656, 100^3 2106.
+constexpr int kSweepBlocks = 4, kProductBlocks = 2;
+// Blocks per SM of the products' grid, which sets the order of their sums; more
+// than are resident, in two even rounds.
+constexpr int kProductGrid = 4;
 
 struct MState {
   KState col[kCols];
@@ -313,7 +317,7 @@ __device__ __forceinline__ void update_alldone(MState *ms) {
 
 // R = B - A X, ||b_l||, ||r_l|| (initial state of every column).
 template <int PA, int KA>
-__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+__global__ void __launch_bounds__(kBlock, kProductBlocks)
     k_mv_init(InfoView<double> a, const double *__restrict__ X,
               const double *__restrict__ B, double *__restrict__ R, MState *ms,
               double *partials) {
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(kBlock, kGatherBlocks)
 
 // Sweep 1 of the apply on all columns: T = D^-1 .* (W^T R).
 template <class V, class T, int PF, int KF>
-__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+__global__ void __launch_bounds__(kBlock, kSweepBlocks)
     k_mv_sweep1(InfoView<V> m, const double *__restrict__ R, const V *__restrict__ d,
                 T *__restrict__ Tm, const MState *ms) {
   if (ms->alldone) return;
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(kBlock, kGatherBlocks)
 
 // Sweep 2 on all columns: Zv = Z T, with rho_l = r_l . z_l and beta_l.
 template <class V, class T, int PF, int KF>
-__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+__global__ void __launch_bounds__(kBlock, kSweepBlocks)
     k_mv_sweep2(InfoView<V> m, const T *__restrict__ Tm, const double *__restrict__ R,
                 double *__restrict__ Zv, MState *ms, double *partials) {
   if (ms->alldone) return;
@@ -420,7 +424,7 @@ __global__ void __launch_bounds__(kBlock)
 
 // Q = A P with sigma_l = p_l . q_l, alpha_l = rho_l / sigma_l.
 template <int PA, int KA>
-__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+__global__ void __launch_bounds__(kBlock, kProductBlocks)
     k_mv_spmm_sigma(InfoView<double> a, const double *__restrict__ P,
                     double *__restrict__ Q, MState *ms, double *partials) {
   if (ms->alldone) return;
@@ -479,7 +483,7 @@ __device__ __forceinline__ bool col_periodic(const KState &c) {
 // Rt = B - A X against R for the columns that need a check; decides
 // confirmation / replacement per column (finish_dots<kTrueRes>).
 template <int PA, int KA>
-__global__ void __launch_bounds__(kBlock, kGatherBlocks)
+__global__ void __launch_bounds__(kBlock, kProductBlocks)
     k_mv_trueres(InfoView<double> a, const double *__restrict__ X,
                  const double *__restrict__ B, const double *__restrict__ R,
                  double *__restrict__ Rt, MState *ms, double *partials) {
@@ -650,17 +654,18 @@ struct ProductLaunch {
   template <int P, int K>
   void run() const {
     const InfoView<double> A = info_view<double>(a);
+    const int grid = std::min((w->n + kBlock - 1) / kBlock, kProductGrid * sm_count());
     if (what == kPInit) {
       auto k = k_mv_init<P, K>;
-      k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(A, w->v(MX), w->v(MB),
+      k<<<grid, kBlock, 0, s>>>(A, w->v(MX), w->v(MB),
                  w->v(MR), w->st, w->partials);
     } else if (what == kPSigma) {
       auto k = k_mv_spmm_sigma<P, K>;
-      k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(A, w->v(MP), w->v(MQ),
+      k<<<grid, kBlock, 0, s>>>(A, w->v(MP), w->v(MQ),
                  w->st, w->partials);
     } else {
       auto k = k_mv_trueres<P, K>;
-      k<<<wave_grid((const void *)k, w->n), kBlock, 0, s>>>(A, w->v(MX), w->v(MB),
+      k<<<grid, kBlock, 0, s>>>(A, w->v(MX), w->v(MB),
                  w->v(MR), w->v(MRT), w->st, w->partials);
     }
   }

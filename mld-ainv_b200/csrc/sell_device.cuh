@@ -730,6 +730,7 @@ inline void launch_dep(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(a)...);
 }
 
+int sm_count();  // of the current device
 // Blocks for kernels that end in a grid-wide reduction: at most one resident
 // wave (8 blocks of 256 threads per SM) so the last block folds few
 // partials; never more blocks than units of 256 rows.

@@ -674,7 +674,6 @@ int stream_plan(const DevSell &m, int xs, int nrv, StreamLayout &L, size_t &smem
 // Slices per consumer warp and stage for a value type (RMAX of stream_rows).
 template <class V>
 constexpr int stream_rmax() { return sizeof(V) >= 8 ? 1 : (int)(8 / sizeof(V)); }
-int sm_count();
 // Allow `bytes` of dynamic shared memory for kernel; false if refused.
 bool set_smem_attr(const void *kernel, size_t bytes);
 
