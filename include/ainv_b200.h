@@ -114,9 +114,10 @@ int ainv_gpu_apply_stage(ainv_handle *h, char trans, int stage, double alpha,
 int ainv_gpu_apply_host(ainv_handle *h, char trans, double alpha, const double *x,
                         double beta, double *y);
 int ainv_gpu_destroy(ainv_handle *h);
-/* Synchronise and report whether any kernel working on h gave up a wait
- * (the streaming kernels bound every wait to about 2 s); clears the flag.
- * AINV_SUCCESS or AINV_ERR_TIMEOUT. */
+/* Synchronise the device and report its errors.  A wait that a kernel gave up
+ * (AINV_ERR_TIMEOUT) is not among them: the calls whose kernels wait on one
+ * another (ainv_gpu_apply_host, ainv_gpu_solve, the solve server) return it
+ * themselves. */
 int ainv_gpu_check(const ainv_handle *h);
 size_t ainv_gpu_sizeof(const ainv_handle *h);
 long long ainv_gpu_get_nzeros(const ainv_handle *h);

@@ -166,7 +166,7 @@ class DeviceFactors:
         return y
 
     def check(self) -> None:
-        """Raise if a device-side wait of a kernel on these factors timed out."""
+        """Synchronise the device; raise if it reports an error."""
         check(lib().ainv_gpu_check(self._h))
 
     def sizeof(self) -> int:
@@ -240,7 +240,7 @@ class DeviceOperator:
         return self._h
 
     def check(self) -> None:
-        """Raise if a device-side wait of a kernel on A timed out."""
+        """Synchronise the device; raise if it reports an error."""
         check(lib().ainv_csr_check(self._h))
 
     def spmv(self, x, y, alpha=1.0, beta=0.0, stream=None) -> None:

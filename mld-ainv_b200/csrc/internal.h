@@ -170,7 +170,6 @@ struct ainv_handle {
   void *t = nullptr;      // intermediate D^-1 W^T x (double for FP64, float otherwise)
   double *xs = nullptr;   // device staging for the host-array apply
   double *ys = nullptr;
-  int *status = nullptr;  // device word: nonzero after a streaming wait timed out
   // host-array apply pipeline: copy-in, sweep and copy-out streams, events,
   // and the schedule for 'N' and 'T'
   cudaStream_t hs[3] = {nullptr, nullptr, nullptr};
@@ -197,7 +196,6 @@ void destroy_host_pipe(HostPipe *hp);
 
 struct ainv_csr {
   int n = 0;
-  int *status = nullptr;  // device word: nonzero after a streaming wait timed out
   ainv::DevSell a;
   ainv::KrylovWs *ws = nullptr;  // Krylov vectors, state and captured graph
   ainv::MrhsWs *mws = nullptr;   // the same for multi-right-hand-side solves

@@ -59,8 +59,7 @@ constexpr int kHistCap = 8192;  // iterations whose residual is recorded
 constexpr int kBarLine = 32, kBarWords = 2 * kBarLine;
 constexpr int kPersistIters = 1024;  // iterations per launch of it
 
-// Where a reduction kernel stores its sums: dot k of group g (or of slice
-// s, for the streaming kernels) at sp[k*ld + g].
+// Where a reduction kernel stores its sums: dot k of slice s at sp[k*ld + s].
 struct SliceOut {
   double *sp;
   int ld, ns;
