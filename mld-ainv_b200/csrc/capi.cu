@@ -368,7 +368,7 @@ int ainv_gpu_destroy(ainv_handle *h) {
 
 size_t ainv_gpu_sizeof(const ainv_handle *h) {
   if (!h) return 0;
-  size_t b = sizeof(*h) + h->wt.bytes() + h->z.bytes() + h->zt.bytes() + h->w.bytes();
+  size_t b = sizeof(*h) + h->wt.bytes + h->z.bytes + h->zt.bytes + h->w.bytes;
   b += ainv::prec_size(h->prec) * (size_t)h->n;                    // D^-1
   b += (h->prec == AINV_PREC_FP32 || h->prec == AINV_PREC_BF16 ? 4 : 8) * (size_t)h->n;  // t
   if (h->xs) b += 2 * sizeof(double) * (size_t)h->n;

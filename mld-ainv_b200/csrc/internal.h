@@ -99,6 +99,7 @@ struct DevSell {
   long long nnz = 0;    // real entries
   long long slots = 0;  // stored values incl. padding
   long long nidx = 0;   // stored index words
+  size_t bytes = 0;     // device memory of all arrays
   int offset_slices = 0;
   int pack = 1;  // P
   int prec = AINV_PREC_FP64;
@@ -111,7 +112,7 @@ struct DevSell {
   // distinct offset lists (a list that several slices share is stored once,
   // so it stays in L1): a kernel that reads a slice through them has every
   // value and gathered element of the slice one load away from its word group.
-  int4 *info = nullptr;  // nslices
+  int4 *info = nullptr;  // nslices; the start of the matrix's one allocation
   int *pidx = nullptr;   // offset lists, each padded to a multiple of P
   int wmax = 0;          // widest slice
   int span = kSlice - 1;  // furthest column a slice reads past its first row (or its last row)
@@ -124,7 +125,6 @@ struct DevSell {
   // host copy: the largest column each slice reads (-1 for an empty slice);
   // a sweep over rows of a slice range needs its input only up to there
   std::vector<int> slice_maxcol;
-  size_t bytes() const;
 };
 
 size_t prec_size(int prec);

@@ -103,11 +103,6 @@ HostCsr transpose(const HostCsr &a) {
   return t;
 }
 
-size_t DevSell::bytes() const {
-  return (size_t)(nslices + 1) * 2 * sizeof(int) + (size_t)nidx * sizeof(int) +
-         (size_t)slots * prec_size(prec);
-}
-
 namespace {
 
 // bfloat16 storage is produced on the host as raw bits: the double is first
@@ -356,6 +351,7 @@ int upload_sell_t(const HostCsr &a, int prec, DevSell &out) {
   const size_t o_idx = part(sizeof(int) * idx.size());
   const size_t o_val = part(sizeof(V) * val.size());
   char *mem = nullptr;
+  m.bytes = total;
   cudaError_t e = cudaMalloc(&mem, total);
   auto fill = [&](size_t at, const void *src, size_t bytes) -> char * {
     if (e == cudaSuccess && bytes)
