@@ -604,7 +604,8 @@ int get_ws(ainv_csr *a, MrhsWs **out) {
   if (e == cudaSuccess) e = cudaMallocHost(&w->hst, sizeof(MState));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMemset(w->mv, 0, sizeof(double) * kNumMv * w->stride);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(w->mv, 0, sizeof(double) * kNumMv * w->stride, w->s);
   if (e != cudaSuccess) {
     destroy_mws(w);
     set_error("block solve workspace allocation failed: %s", cudaGetErrorString(e));

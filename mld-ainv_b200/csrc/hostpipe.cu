@@ -307,7 +307,8 @@ int host_pipe_apply(ainv_handle *h, bool tr, const HostPlan &p, double alpha, co
     hp.cap = 0;
     AINV_CUDA_TRY(cudaMalloc(&hp.ctr, sizeof(int) * (size_t)(C + 2)));
     AINV_CUDA_TRY(cudaMalloc(&hp.flags, sizeof(unsigned) * (size_t)C));
-    AINV_CUDA_TRY(cudaMemset(hp.flags, 0, sizeof(unsigned) * (size_t)C));
+    AINV_CUDA_TRY(cudaMemsetAsync(hp.flags, 0, sizeof(unsigned) * (size_t)C, si));
+    AINV_CUDA_TRY(cudaStreamSynchronize(si));
     hp.cap = C;
     hp.epoch = 0;
   }
@@ -325,6 +326,7 @@ int host_pipe_apply(ainv_handle *h, bool tr, const HostPlan &p, double alpha, co
                              cudaMemcpyHostToDevice));
     AINV_CUDA_TRY(cudaMemcpy(it.pieces1, pieces1.data(), sizeof(int) * pieces1.size(),
                              cudaMemcpyHostToDevice));
+    AINV_CUDA_TRY(cudaStreamSynchronize(nullptr));  // the copies may still be under way
     it.nitems = (int)items.size();
     it.C = C;
     it.cs = p.cs;

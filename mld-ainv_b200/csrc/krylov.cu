@@ -462,7 +462,6 @@ int get_ws(ainv_csr *a, KrylovWs **out) {
   const size_t hist = part(sizeof(double) * kHistCap);
   const size_t bar = part(sizeof(unsigned) * kBarWords), loop = part(sizeof(LoopState));
   cudaError_t e = cudaMalloc(&w->mem, at);
-  if (e == cudaSuccess) e = cudaMemset(w->mem, 0, at);
   w->vec = reinterpret_cast<double *>(w->mem + vec);
   w->sp = reinterpret_cast<double *>(w->mem + sp);
   w->rs = reinterpret_cast<double *>(w->mem + rs);
@@ -476,6 +475,7 @@ int get_ws(ainv_csr *a, KrylovWs **out) {
   w->hst = &w->hloop->k;
   w->hist_h = reinterpret_cast<double *>(w->hmem + hh);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemsetAsync(w->mem, 0, at, w->s);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     destroy_ws(w);
@@ -777,7 +777,7 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
       AINV_CUDA_TRY(cudaStreamSynchronize(w->s));
       if (w->hloop->abort) {
         w->hst->timeout = 1;
-        AINV_CUDA_TRY(cudaMemset(w->bar, 0, sizeof(unsigned) * kBarWords));
+        AINV_CUDA_TRY(cudaMemsetAsync(w->bar, 0, sizeof(unsigned) * kBarWords, w->s));
       }
       if (w->hst->done || w->hst->timeout) {
         AINV_CUDA_TRY(cudaEventRecord(w->ev, w->s));

@@ -366,6 +366,9 @@ int upload_sell_t(const HostCsr &a, int prec, DevSell &out) {
   m.iptr = reinterpret_cast<int *>(fill(o_iptr, iptr.data(), sizeof(int) * iptr.size()));
   m.idx = reinterpret_cast<int *>(fill(o_idx, idx.data(), sizeof(int) * idx.size()));
   m.val = fill(o_val, val.data(), sizeof(V) * val.size());
+  // a copy from pageable memory may return while it is under way, and streams
+  // that do not wait for the default one read the matrix
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e != cudaSuccess) {
     free_sell(m);
     set_error("device upload of sliced matrix failed: %s", cudaGetErrorString(e));
@@ -416,6 +419,7 @@ int upload_values(const double *h, size_t n, int prec, void **dptr) {
   }
   cudaError_t e = cudaMalloc(dptr, n * es);
   if (e == cudaSuccess) e = cudaMemcpy(*dptr, buf.data(), n * es, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // as for a matrix
   if (e != cudaSuccess) {
     if (*dptr) cudaFree(*dptr);
     *dptr = nullptr;

@@ -1814,10 +1814,10 @@ int ainv_server_create(ainv_server **out, int max_slots, size_t hbm_bytes, int i
     return fail(e, "states");
   if ((e = cudaMalloc(&srv->bars, sizeof(unsigned) * kBarWords)) != cudaSuccess)
     return fail(e, "counters");
-  if ((e = cudaMemset(srv->bars, 0, sizeof(unsigned) * kBarWords)) != cudaSuccess)
-    return fail(e, "counters");
   if ((e = cudaStreamCreateWithFlags(&srv->s, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(e, "stream");
+  if ((e = cudaMemsetAsync(srv->bars, 0, sizeof(unsigned) * kBarWords, srv->s)) != cudaSuccess)
+    return fail(e, "counters");
   std::memset(srv->tab_h, 0, sizeof(Table));
   std::fill(srv->tab_h->block_slot, srv->tab_h->block_slot + kMaxGrid, (short)-1);
   std::fill(srv->tab_h->block_slot_f, srv->tab_h->block_slot_f + kMaxGrid, (short)-1);
