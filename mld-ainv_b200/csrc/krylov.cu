@@ -705,9 +705,22 @@ int persist_prec(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const dou
   }
 }
 
+bool narrow_factors(const ainv_handle *h) { return h->wt.wmax <= 4 && h->z.wmax <= 4; }
+
+// Whether a solve runs there: few enough groups per team for its rows' slots.
+bool persist_fits(const KrylovWs *w, const ainv_handle *h, const ainv_csr *a) {
+  const int teams = kPTeams * 2 * sm_count();
+  const long long rounds = (w->ng + teams - 1) / teams, rows = (long long)w->ns * kSlice;
+  const int p = fast_pack(prec_size(h->prec), narrow_factors(h));
+  const bool fast = h->wt.pack == p && h->z.pack == p && a->a.pack == 1;
+  return w->n <= kPMaxRows && rounds <= kPMaxPerTeam &&
+         rounds * (h->wt.slots + h->z.slots) <= persist_limit(h->prec, fast) * rows &&
+         rounds * a->a.slots <= kPMaxASlots * rows;
+}
+
 int persist(KrylovWs *w, const ainv_handle *h, const ainv_csr *a, const double *b, double *x,
             int method, int resume) {
-  const bool narrow = h->wt.wmax <= 4 && h->z.wmax <= 4;
+  const bool narrow = narrow_factors(h);
   if (method == AINV_KRYLOV_CG)
     return narrow ? persist_prec<4, AINV_KRYLOV_CG>(w, h, a, b, x, resume)
                   : persist_prec<8, AINV_KRYLOV_CG>(w, h, a, b, x, resume);
@@ -762,9 +775,7 @@ int krylov_solve(const ainv_handle *h, ainv_csr *a, const double *b, double *x, 
   init.hist_cap = kHistCap;
   *w->hloop = LoopState{init, 0};
   AINV_CUDA_TRY(cudaMemcpyAsync(w->loop, w->hloop, sizeof(LoopState), cudaMemcpyHostToDevice, w->s));
-  const bool persistent =
-      h && n <= kPMaxRows && w->ng <= kPMaxPerTeam * kPTeams * 2 * sm_count();
-  if (persistent) {
+  if (h && persist_fits(w, h, a)) {
     for (int resume = 0;; resume = 1) {
       const int rc = persist(w, h, a, b, x, method, resume);
       if (rc == AINV_ERR_UNSUPPORTED && !resume) break;  // no cooperative launch: plain loop

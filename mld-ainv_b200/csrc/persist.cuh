@@ -52,9 +52,30 @@ constexpr int kPWarps = kPBlock / 32;
 // the bytes it moves, and the plain kernels, with 48 warps per SM against 32,
 // move them faster: us per iteration here / there at 52^3 CG 15.1 / 28.6,
 // 64^3 CG 20.0 / 34.0, 64^3 BiCGSTAB 35.4 / 52.3 (2 groups), 80^3 CG 37.4 /
-// 42.9, 80^3 BiCGSTAB 69.8 / 72.3 (4 groups), 90^3 BiCGSTAB 92.9 / 85.9,
-// 100^3 BiCGSTAB 120 / 112.
+// 42.9, 84^3 BiCGSTAB 81.7 / 85.4 (4 groups), 90^3 BiCGSTAB 92.9 / 85.9,
+// 100^3 BiCGSTAB 120 / 112.  These have factors of 4 slots and an A of 7; wider
+// ones end earlier (persist_limit).
 constexpr int kPMaxPerTeam = 4;
+// Limits on slots per row times groups per team, for both factors together and
+// for A.  A phase takes a row's slots 8 at a time one after the other, with up
+// to three gathers per slot and registers that spill, so that wide rows cost
+// here what the launches cost there; how much depends on the values' loads
+// (fast: the packs with kernels of their own).  us per iteration here / there,
+// the last size kept and the first one left to the plain loop:
+//   INVK(1,1), 23 slots: FP64 BiCGSTAB 52^3 (1 group) 43.7 / 58.5, 60^3 (2) 87.6 /
+//   78.8; FP32 66^3 (2) 68.3 / 78.8, 69^3 (3) 91.3 / 85.0; FP32_ACC64 63^3 (2) 68.3 /
+//   73.5, 69^3 98.2 / 83.4; BF16_ACC64 fast 66^3 (2) 68.0 / 75.3, 69^3 88.2 / 77.8,
+//   not fast (56^3: the rows' average is 22) 94.4 / 59.9; BF16 not fast 52^3 (1) 54.4 /
+//   57.8, 56^3 (2) 87.1 / 60.3.
+//   11 slots, not fast: FP64 CG 84^3 (4) 80.9 / 83.3; FP32_ACC64 72^3 (3) 67.6 / 68.5,
+//   84^3 (4) 115 / 83.1.
+//   131 slots, not fast: FP64 BiCGSTAB 20^3 137 / 101, 46^3 254 / 178.
+//   A of 27 slots with factors of 1: CG 66^3 (2) 44.4 / 50.7, 68^3 (3) 57.9 / 52.9.
+constexpr int kPMaxASlots = 56;
+constexpr int persist_limit(int prec, bool fast) {
+  if (fast) return prec == AINV_PREC_FP64 ? 64 : 96;
+  return prec == AINV_PREC_BF16_ACC64 ? 44 : prec == AINV_PREC_FP32_ACC64 ? 66 : 88;
+}
 // Ranges a block folds in one step (one lane each): 32 ranges of 256 groups.
 constexpr int kPMaxRanges = 32;
 constexpr long long kPMaxRows = (long long)kPMaxRanges * kFoldRange * kGroupSlices * kSlice;
@@ -715,11 +736,14 @@ struct PLoop {
   }
 };
 
-// The pack that most matrices of a width class get (layout.cpp), the one with
-// kernels of its own.
+// The pack that most matrices of a width class (at most 4 slots, or more) get
+// (layout.cpp), the one with kernels of its own.
+constexpr int fast_pack(size_t value_bytes, bool narrow) {
+  return value_bytes == 8 ? 2 : value_bytes == 4 || narrow ? 4 : 8;
+}
 template <class V, int K>
 constexpr int fast_pack() {
-  return sizeof(V) == 8 ? 2 : sizeof(V) == 4 || K <= 4 ? 4 : 8;
+  return fast_pack(sizeof(V), K <= 4);
 }
 
 // One solve (or max_iters iterations of it) by the whole grid.
