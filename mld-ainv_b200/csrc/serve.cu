@@ -895,6 +895,21 @@ constexpr int kPersistBlocks = 2;  // per SM
 // 16.7, 16 of 64^3 (27.7) 26.7 / 27.3; past that the two are level, and the
 // batched kernels share an operator's reads.
 constexpr int kPersistPerTeam = 32;
+// Limits on slots per row times groups per team (summed over the mix) for A and,
+// where factors have more than 4 slots, for both factors together: the members
+// of a group each read the operator's words here, and rows are taken 8 slots at
+// a time (persist_limit of the single solve).  Batch times here / there in ms:
+//   A of 27 slots, factors of 1: 4 of 64^3 (6.9 groups) 8.2 / 8.6, 8 (13.8) 15.4 / 14.4.
+//   INVK(1,1), 23 slots: FP64 3 of 80^3 (10.1) 23.8 / 24.5, 2 of 100^3 (13.2) 40.8 /
+//   38.2; FP32 18.8 / 19.9, 4 of 80^3 (13.5) 24.3 / 23.5; BF16 2 of 80^3 (6.8) 13.3 /
+//   13.6, 3 18.1 / 17.1; BF16_ACC64 4 of 40^3 (1.7) 4.7 / 6.6, 1 of 80^3 (3.4) 10.1 / 9.9.
+//   11 slots, packs without kernels of their own: FP64 4 of 64^3 1.71 / 1.96, 8 3.14 /
+//   3.00; FP32_ACC64 8 of 40^3 (3.4) 1.20 / 1.85, 4 of 64^3 2.20 / 2.05.
+constexpr int kPersistASlots = 224;
+constexpr int persist_mix_limit(int prec, bool fast) {
+  if (fast) return prec == AINV_PREC_BF16_ACC64 ? 150 : prec == AINV_PREC_BF16 ? 320 : 512;
+  return prec == AINV_PREC_FP32_ACC64 || prec == AINV_PREC_BF16_ACC64 ? 100 : 200;
+}
 // Arrival counters: [parity][slot], on lines of their own.
 constexpr int kBarLine = 32;
 constexpr int kBarWords = 2 * kMaxSlots * kBarLine;
@@ -956,25 +971,21 @@ __global__ void __launch_bounds__(kPBlock, kPersistBlocks)
 
 // The kernel for a precision; narrow: factor slices of at most 4 slots; fast:
 // the packs that have kernels of their own.
-template <class V, class T, int K>
-void *persist_kernel_k(bool fast) {
-  return fast ? (void *)k_srv_persist<V, T, fast_pack<V, K>(), K> : (void *)k_srv_persist<V, T, 0, K>;
-}
 template <class V, class T>
-void *persist_kernel_v(bool narrow, const SlotDesc *const *d, size_t n) {
-  const int P = narrow ? fast_pack<V, 4>() : fast_pack<V, 8>();
-  bool fast = true;
-  for (size_t q = 0; q < n; q++)
-    fast = fast && d[q]->wt.pack == P && d[q]->z.pack == P && d[q]->A.pack == 1;
-  return narrow ? persist_kernel_k<V, T, 4>(fast) : persist_kernel_k<V, T, 8>(fast);
+void *persist_kernel_v(bool narrow, bool fast) {
+  if (narrow)
+    return fast ? (void *)k_srv_persist<V, T, fast_pack<V, 4>(), 4>
+                : (void *)k_srv_persist<V, T, 0, 4>;
+  return fast ? (void *)k_srv_persist<V, T, fast_pack<V, 8>(), 8>
+              : (void *)k_srv_persist<V, T, 0, 8>;
 }
-void *persist_kernel(int prec, bool narrow, const SlotDesc *const *d, size_t n) {
+void *persist_kernel(int prec, bool narrow, bool fast) {
   switch (prec) {
-    case AINV_PREC_FP64: return persist_kernel_v<double, double>(narrow, d, n);
-    case AINV_PREC_FP32: return persist_kernel_v<float, float>(narrow, d, n);
-    case AINV_PREC_BF16: return persist_kernel_v<__nv_bfloat16, float>(narrow, d, n);
-    case AINV_PREC_FP32_ACC64: return persist_kernel_v<f32w, double>(narrow, d, n);
-    case AINV_PREC_BF16_ACC64: return persist_kernel_v<b16w, double>(narrow, d, n);
+    case AINV_PREC_FP64: return persist_kernel_v<double, double>(narrow, fast);
+    case AINV_PREC_FP32: return persist_kernel_v<float, float>(narrow, fast);
+    case AINV_PREC_BF16: return persist_kernel_v<__nv_bfloat16, float>(narrow, fast);
+    case AINV_PREC_FP32_ACC64: return persist_kernel_v<f32w, double>(narrow, fast);
+    case AINV_PREC_BF16_ACC64: return persist_kernel_v<b16w, double>(narrow, fast);
   }
   return nullptr;
 }
@@ -1498,29 +1509,42 @@ void fill_slot(ainv_server *srv, int k, const Request *r, size_t off) {
 
 // Whether the admitted slots run in the persistent loop, and their blocks
 // there: one precision, every matrix within the loop's rows, and no more
-// groups than kPersistPerTeam per team.
+// groups per team than the limits above.
 void plan_persist(ainv_server *srv, const std::vector<int> &order) {
   srv->persist = nullptr;
   if (order.empty()) return;
   const int grid = std::min(kMaxGrid, kPersistBlocks * sm_count());
   if ((int)order.size() > grid) return;
   const SlotDesc &first = srv->tab_h->slot[order[0]];
+  const int prec = first.wt.prec;
   const bool narrow = first.wt.wmax <= 4 && first.z.wmax <= 4;
-  long long groups = 0;
+  const int pack = fast_pack(prec_size(prec), narrow);
+  bool fast = true;
+  double groups = 0.0, fslots = 0.0, aslots = 0.0;  // per team
+  double fmax = 0.0, amax = 0.0;                    // of one group
+  const double teams = (double)kPTeams * grid;
   std::vector<long long> w(order.size());
   std::vector<int> cap(order.size()), b0(order.size()), nb(order.size());
-  std::vector<const SlotDesc *> descs(order.size());
   for (size_t q = 0; q < order.size(); q++) {
     const SlotDesc &d = srv->tab_h->slot[order[q]];
-    descs[q] = &d;
-    if (d.smask || d.wt.prec != first.wt.prec || d.n > kPMaxRows ||
+    const Operator &op = srv->slots[(size_t)order[q]].req->opd;
+    if (d.smask || d.wt.prec != prec || d.n > kPMaxRows ||
         (d.wt.wmax <= 4 && d.z.wmax <= 4) != narrow)
       return;
-    groups += d.ng;
+    fast = fast && d.wt.pack == pack && d.z.pack == pack && d.A.pack == 1;
+    const double rows = (double)d.ns * kSlice;
+    const double fs = (double)(op.h->wt.slots + op.h->z.slots) / rows;
+    const double as = (double)op.a->a.slots / rows;
+    groups += d.ng / teams;
+    fslots += fs * d.ng / teams;
+    aslots += as * d.ng / teams;
+    fmax = std::max(fmax, fs);
+    amax = std::max(amax, as);
     w[q] = d.ng;
     cap[q] = (d.ng + kPTeams - 1) / kPTeams;
   }
-  if (groups > (long long)kPersistPerTeam * kPTeams * grid) return;
+  if (groups > kPersistPerTeam || std::max(aslots, amax) > kPersistASlots) return;
+  if (!narrow && std::max(fslots, fmax) > persist_mix_limit(prec, fast)) return;
   if (plan_weighted((int)order.size(), w.data(), cap.data(), grid, b0.data(), nb.data()) !=
       AINV_SUCCESS)
     return;
@@ -1531,7 +1555,7 @@ void plan_persist(ainv_server *srv, const std::vector<int> &order) {
     d.pnb = nb[q];
     for (int b = d.pb0; b < d.pb0 + d.pnb; b++) srv->tab_h->block_slot_p[b] = (short)order[q];
   }
-  srv->persist = persist_kernel(first.wt.prec, narrow, descs.data(), descs.size());
+  srv->persist = persist_kernel(prec, narrow, fast);
 }
 
 // One launch of the persistent loop; false (and the graph from then on, until

@@ -72,3 +72,30 @@ def test_solve(monkeypatch, points, factors, idim, prec, persistent):
             assert (got.info, got.iter, got.err) == (want.info, want.iter, want.err)
             assert torch.equal(x, y)
         monkeypatch.delenv("AINV_WAIT_MS")
+
+
+@pytest.mark.parametrize("points,factors,idim,prec,persistent", [
+    (7, "AINV", 24, "FP32", True), (7, "INVK", 40, "FP64", True),
+    (7, "INVK", 50, "BF16_ACC64", True), (7, "INVK", 86, "BF16_ACC64", False),
+    (3, "AINV", 80, "FP32_ACC64", True), (3, "AINV", 90, "FP32_ACC64", False),
+    (27, "AINV", 50, "FP64", True), (27, "INVK", 20, "FP64", False),
+])
+def test_server(monkeypatch, points, factors, idim, prec, persistent):
+    """One request, so that it is the whole mix."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are for 148 multiprocessors")
+    A, f = system(points, factors, idim, prec)
+    b = np.random.default_rng(0).uniform(-1, 1, idim ** 3)
+    x = torch.zeros(idim ** 3, dtype=torch.float64, device="cuda")
+    assert A.solve(torch.from_numpy(b).cuda(), x, f, "BICGSTAB", 1e-6, 200).converged
+    y = np.zeros_like(b)
+    monkeypatch.setenv("AINV_WAIT_MS", "0")
+    with ainv.SolveServer(max_slots=2, hbm_bytes=1 << 30) as srv:
+        i = srv.submit(srv.add_operator(A, f), b, y, 1e-6, 200)
+        if persistent:
+            with pytest.raises(ainv.AinvError) as e:
+                srv.wait(i, timeout=60.0)
+            assert e.value.info == TIMEOUT and "time limit" in str(e.value)
+        else:
+            assert srv.wait(i, timeout=60.0).converged
+            assert np.array_equal(y, x.cpu().numpy())
