@@ -35,9 +35,9 @@ using namespace dev;
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
     k_sweep_dscale(InfoView<V> m, const double *x, const V *d, T *t, int s0, int s1,
-                   const volatile int *stop) {
+                   const int *stop) {
   for_each_info<P, K>(
-      m, x, s0, s1, [&] { return !stop || !*stop; }, [&](int row) { return ldd_now(d + row); },
+      m, x, s0, s1, [&] { return !stop || !ld_now(stop); }, [&](int row) { return ldd_now(d + row); },
       [&](int row, auto acc, auto dr) { t[row] = (T)(dr * acc); }, [](int) {});
 }
 
@@ -46,9 +46,9 @@ __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
     k_sweep_axpby(InfoView<V> m, const T *t, double alpha, double beta, double *y, int s0, int s1,
-                  const volatile int *stop) {
+                  const int *stop) {
   for_each_info<P, K>(
-      m, t, s0, s1, [&] { return !stop || !*stop; },
+      m, t, s0, s1, [&] { return !stop || !ld_now(stop); },
       [&](int row) { return beta == 0.0 ? 0.0 : ld_now(y + row); },
       [&](int row, auto acc, double yr) { y[row] = axpby_row(alpha, (double)acc, beta, yr); },
       [](int) {});

@@ -53,6 +53,11 @@ __device__ __forceinline__ float ld_now(const float *p) {
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ int ld_now(const int *p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ unsigned ld_now(const unsigned short *p) {
   unsigned short v;
   asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
