@@ -164,7 +164,14 @@ int ainv_csr_check(const ainv_csr *a);
  * x_dev holds x0 on entry and the solution on exit; h may be NULL (no
  * preconditioner).  Returns AINV_SUCCESS on convergence, AINV_ERR_NOCONV
  * at itmax, AINV_ERR_BREAKDOWN / AINV_ERR_NONFINITE on breakdown; *iter and
- * *err (relative residual) are set in every case. */
+ * *err (relative residual) are set in every case.
+ * A small system with a preconditioner (up to about 600,000 rows, fewer with
+ * wide factors) runs as one cooperative kernel whose blocks wait for one
+ * another: it holds every multiprocessor until it ends, or for 1024 iterations
+ * at a time, so such solves from several threads, or beside a solve server,
+ * take turns on the GPU.  Where a block waits longer than 2 s (AINV_WAIT_MS
+ * milliseconds, read per call) the solve ends with AINV_ERR_TIMEOUT and x_dev
+ * is not the solution; the next solve on the same objects starts afresh. */
 int ainv_gpu_solve(ainv_handle *h, const ainv_csr *a, const double *b_dev,
                    double *x_dev, int method, double eps, int itmax, int *iter,
                    double *err, void *stream);
@@ -280,7 +287,8 @@ typedef struct ainv_server ainv_server;
 typedef struct {
   long long id;
   int op;          /* operator index from ainv_server_add_operator */
-  int status;      /* AINV_SUCCESS, AINV_ERR_NOCONV, ... as ainv_gpu_solve */
+  int status;      /* AINV_SUCCESS, AINV_ERR_NOCONV, ... as ainv_gpu_solve;
+                      AINV_ERR_TIMEOUT if a device wait for it was given up */
   int iter;        /* BiCGSTAB iterations */
   double err;      /* final relative residual (confirmed on b - A x) */
   double t_submit; /* server clock (seconds since creation) */
@@ -298,8 +306,10 @@ typedef struct {
 /* max_slots (1..64): requests in flight together.  hbm_bytes: device bytes
  * for the requests' vectors (0: half of the free HBM); a request is admitted
  * only while its vectors fit (ainv_server_request_bytes).  iters_per_launch
- * (1..64): iterations per graph launch, i.e. how often completion is
- * checked.  Starts the server's engine thread on the current device. */
+ * (1..64): iterations per launch, i.e. how often completion is checked.
+ * Small mixes run as one cooperative kernel per launch, which holds every
+ * multiprocessor for those iterations; AINV_WAIT_MS as in ainv_gpu_solve, read
+ * here.  Starts the server's engine thread on the current device. */
 int ainv_server_create(ainv_server **srv, int max_slots, size_t hbm_bytes,
                        int iters_per_launch);
 /* Register a resident operator A with its factors h (AINV, INVK or INVT,
@@ -314,7 +324,8 @@ int ainv_server_submit(ainv_server *srv, int op, const double *b, double *x, dou
                        int itmax, long long *id);
 /* Wait for request id (timeout_s < 0: no limit); fills *res (may be NULL)
  * and returns the request's status, or AINV_ERR_TIMEOUT if it is still
- * running.  Each id is waited for once. */
+ * running (*res is then left as it was; a request that itself ended with that
+ * status fills it).  Each id is waited for once. */
 int ainv_server_wait(ainv_server *srv, long long id, double timeout_s, ainv_result *res);
 int ainv_server_stats(ainv_server *srv, ainv_server_info *out);
 /* Finishes every queued request, stops the engine, frees the server. */

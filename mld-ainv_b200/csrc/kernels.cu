@@ -30,8 +30,8 @@ namespace {
 using namespace dev;
 
 // Slices [s0, s1) of a sweep (all of them, or a range of the host-array
-// pipeline).  HBM-bound: at 200^3 in FP64 sweep 1 moves 453 MB in 70.4 us and
-// sweep 2 389 MB in 60.7 us, 6.4 TB/s each.
+// pipeline).  HBM-bound: at 200^3 in FP64 sweep 1 moves 453 MB and sweep 2 389 MB,
+// together in 134-140 us on different boards, 6.0-6.3 TB/s (a copy: 6.5).
 template <class V, class T, int P, int K>
 __global__ void __launch_bounds__(kBlock, info_blocks<V, K>())
     k_sweep_dscale(InfoView<V> m, const double *x, const V *d, T *t, int s0, int s1,

@@ -450,11 +450,10 @@ __device__ __forceinline__ void group_dot(const SellView<V> &m, const GroupCtx<S
 // summed) stands between a warp and all of a slice's values and gathered
 // elements.  The chain slice pointers -> offsets -> gathers of group_dot,
 // three DRAM round trips per step, held the sweeps at 4.5-4.9 TB/s; these
-// run at the copy peak (200^3 FP64: sweep 1 90.3 -> 70.4 us, sweep 2 79.9 ->
-// 60.7 us, 6.4 TB/s each) and beat the bulk-copy pipeline of stream.cuh at
-// every precision and pattern measured (128^3 FP32 40.6 -> 30.8 us per apply,
-// 101^3 BF16 26.8 -> 18.3, 100^3 INVK FP64 83.7 -> 71.4, 128^3 scattered
-// columns FP64 82.3 -> 70.9).
+// run near a copy's rate (200^3 FP64 apply 172.5 -> 139.7 us, 6.0 TB/s) and beat
+// the bulk-copy pipeline of stream.cuh at every precision and pattern measured
+// (128^3 FP32 40.6 -> 30.8 us per apply, 101^3 BF16 26.8 -> 18.3, 100^3 INVK
+// FP64 83.7 -> 71.4, 128^3 scattered columns FP64 82.3 -> 70.9).
 template <class V>
 struct InfoView {
   int n, nslices;
